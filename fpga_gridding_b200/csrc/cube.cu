@@ -220,6 +220,7 @@ int cube_build(oskar_B200Cube* c, const void* d_conv, const void* d_conv_im,
         if (d.bytes > max_bytes) max_bytes = d.bytes;
     }
     c->max_slab_bytes = max_bytes;
+    c->group_support = assign_groups(c->planes.data(), P);
     cudaError_t e = c->d_planes.ensure(sizeof(PlaneDesc) * P);
     if (e == cudaSuccess) e = c->d_slabs.ensure((size_t)off * c->elem_bytes);
     if (e == cudaSuccess)
@@ -306,7 +307,7 @@ int cube_build(oskar_B200Cube* c, const void* d_conv, const void* d_conv_im,
 // gives), for callers that place the re-laid cube in memory they provide.
 size_t static_cube_geometry(int num_planes, const int* support,
                             int oversample, std::vector<PlaneDesc>* planes,
-                            unsigned* max_block_bytes)
+                            unsigned* max_block_bytes, int* num_groups)
 {
     const int half = (oversample + 1) / 2;
     const int elem = (int)sizeof(float2);
@@ -330,6 +331,7 @@ size_t static_cube_geometry(int num_planes, const int* support,
         off += (long long)elems;
     }
     *max_block_bytes = max_block;
+    *num_groups = (int)assign_groups(planes->data(), num_planes).size();
     return (size_t)off * elem;
 }
 

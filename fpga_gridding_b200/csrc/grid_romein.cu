@@ -1,8 +1,8 @@
 // Romein-style W-projection scatter kernel for sm_100a.
 //
 // Work arrives as tasks: runs of <= kTaskMax sorted visibilities that share
-// a w-plane (hence a support S and footprint width W = 2S+1) and a coarse
-// grid tile.  A persistent CTA pulls tasks from a device work queue.  For a
+// a support S (hence a footprint width W = 2S+1) and a coarse grid tile; with
+// staging on, a w-plane.  A persistent CTA pulls tasks from a device work queue.  For a
 // task it
 //   0. gathers the task's placement records and visibilities through the
 //      sort's index array (sorted position -> point),
@@ -22,6 +22,7 @@
 //   grid[v][u] += vis * (conj ? conj(K) : K)(|off_v + j*os|, |off_u + k*os|)
 // (oskar_grid_wproj.c:104-123), summed in a different order.
 #include <algorithm>
+#include <climits>
 #include <mutex>
 #include <type_traits>
 
@@ -39,14 +40,18 @@ template <> struct Vec2<double> { using type = double2; };
 // Per-visibility tap record.  For a class (a, b) of a task with footprint W:
 //   ru = (a + mu) mod W, rv = (b + mv) mod W   (offsets inside the footprint)
 //   column = ru >= tu ? cp + ru : cn - ru      (slab column, see PlaneDesc)
-//   kernel index = rowbase + column + rv * pitch
+//   kernel index = base + column + rv * pitch
 //   cell         = origin + ru + rv * grid_size
+// base: L1 path, the address of the visibility's first slab row (the points
+// of a task may lie on several planes of one support); staged path, the index
+// of that row in the plane's slab.
 template <typename GT>
 struct __align__(16) TapVis
 {
     unsigned origin;
     int mu, mv, tu;
-    int cp, cn, rowbase, unused;
+    int cp, cn;
+    long long base;
     // re += c0.x * Kre + c1.x * Kim;  im += c0.y * Kre + c1.y * Kim
     typename Vec2<GT>::type c0, c1;
 };
@@ -81,10 +86,12 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 c0,
     acc.y = fma(c1.y, k.y, acc.y);
 }
 
-template <typename GT>
+// slabs: the cube's slab array (L1 path), or null (staged path).
+template <typename GT, typename KT>
 __device__ __forceinline__ TapVis<GT> derive(const int4 rec,
                                              const typename Vec2<GT>::type vis,
-                                             const PlaneDesc& d, int grid_size,
+                                             const PlaneDesc& d,
+                                             const KT* slabs, int grid_size,
                                              int oversample, int half,
                                              unsigned long long* status)
 {
@@ -106,8 +113,8 @@ __device__ __forceinline__ TapVis<GT> derive(const int4 rec,
     t.cp = rpu * d.L + (off_u - rpu) / os - s;
     t.cn = rnu * d.L + (-off_u - rnu) / os + s;
     // First of the W slab rows holding this row offset's taps.
-    t.rowbase = (off_v + half) * w * d.pitch;
-    t.unused = 0;
+    const int row = (off_v + half) * w * d.pitch;
+    t.base = slabs ? (long long)(slabs + d.offset + row) : (long long)row;
     GT sc = (GT)d.scale;
     // The prep kernel only keeps points whose footprint lies inside the
     // grid; a record that breaks this is reported and neutralised (zero
@@ -138,42 +145,89 @@ __device__ __forceinline__ uint32_t spread9(uint32_t x)
     return x;
 }
 
-// Layout of the in-task order key, most significant first:
+// In-task order key, most significant first:
 //   row-offset major (staged kernel values: each row offset's run reads one
 //   W-row block):  (off_v + H) | Morton(gu, gv) | (off_u + H) | index
-//   cell major (kernel values through L1):  Morton(gu, gv) | (off_v + H) |
-//   (off_u + H) | index.  Neighbouring visibilities then share most class
-//   cells, which halves the grid atomics at plain_large (6.6e9 -> 3.4e9)
-//   and is 1.7 % faster there than row-offset major.
+//   cell major (kernel values through L1):  column gu | row gv (up and down
+//   in turn) | low bits of the w-plane | (off_v + H) | (off_u + H) | index.
+//   Neighbours then mostly differ in gv: what leaves their shared footprint
+//   is whole rows, which a warp adds to the grid as contiguous lanes, while a
+//   step in gu flushes one lane of every row.  Against Morton order of the
+//   same tasks: plain_large gridding 16.6 -> 16.3 ms, a 10x thinner one
+//   2.15 -> 2.12 ms.
 // The offsets take `ob` bits each (the bit width of 2H, H = ceil(os / 2)),
-// the index the low 8 bits, and the Morton code of the low `mb` (<= 9) bits
-// of gu and gv what is left.  Records with identical taps are adjacent in
-// either order.
+// the index the low 8 bits.  Cell major: column and row are counted from the
+// task's smallest ones, so they need only the bits of its extent; what is
+// left over tells planes apart (at least 3 bits; the row's low bits are
+// dropped where they do not fit).  Records with identical taps are adjacent,
+// except where more planes meet in a cell than those bits can tell apart.
 struct TaskKey
 {
-    int ob, mb;
-    bool cell_major;
-    __device__ __forceinline__ TaskKey(int half, bool cell_major_order)
+    int ob, mb;           // row-offset major
+    int u0, v0, bv, pb, shift;
+    // box: smallest and largest gu (x, y) and gv (z, w) of the task
+    __device__ __forceinline__ TaskKey(int half, const int4 box)
     {
         ob = 32 - __clz(2 * half);
-        mb = min(9, (32 - 8 - 2 * ob) / 2);
-        cell_major = cell_major_order;
+        const int avail = 32 - 8 - 2 * ob;
+        mb = min(9, avail / 2);
+        u0 = box.x;
+        v0 = box.z;
+        bv = 32 - __clz(box.w - box.z);
+        const int bits = 32 - __clz(box.y - box.x) + bv;
+        pb = min(max(avail - bits, 3), 15);
+        shift = max(bits + pb - avail, 0);
     }
+    template <bool CELL_MAJOR>
     __device__ __forceinline__ uint32_t make(const int4 r, unsigned t) const
     {
-        const uint32_t mask = (1u << mb) - 1u;
-        const uint32_t morton = spread9((uint32_t)r.x & mask) |
-                                (spread9((uint32_t)r.y & mask) << 1);
         const uint32_t ov = (uint32_t)(r.w >> 16), ou = (uint32_t)(r.w & 0xffff);
-        if (cell_major)
-            return (morton << (8 + 2 * ob)) | (ov << (8 + ob)) | (ou << 8) | t;
-        return (ov << (32 - ob)) | (morton << (8 + ob)) | (ou << 8) | t;
+        if constexpr (CELL_MAJOR)
+        {
+            const uint32_t du = (uint32_t)(r.x - u0);
+            uint32_t dv = (uint32_t)(r.y - v0);
+            if (du & 1u) dv = (1u << bv) - 1u - dv;
+            const uint32_t plane = (uint32_t)r.z & ((1u << pb) - 1u);
+            return ((((((du << bv | dv) >> shift) << pb | plane) << ob | ov)
+                     << ob | ou) << 8) | t;
+        }
+        else
+        {
+            const uint32_t mask = (1u << mb) - 1u;
+            const uint32_t morton = spread9((uint32_t)r.x & mask) |
+                                    (spread9((uint32_t)r.y & mask) << 1);
+            return (ov << (32 - ob)) | (morton << (8 + ob)) | (ou << 8) | t;
+        }
     }
     __device__ __forceinline__ int row_offset(uint32_t key) const
     {
         return (int)(key >> (32 - ob));
     }
 };
+
+// Smallest and largest gu (x, y) and gv (z, w) of a task's records (`in`:
+// this thread holds one).  All threads of the CTA must call it.
+__device__ __forceinline__ int4 task_box(bool in, const int4 rec, int4* s_box)
+{
+    const int x0 = __reduce_min_sync(0xffffffffu, in ? rec.x : INT_MAX);
+    const int x1 = __reduce_max_sync(0xffffffffu, in ? rec.x : INT_MIN);
+    const int y0 = __reduce_min_sync(0xffffffffu, in ? rec.y : INT_MAX);
+    const int y1 = __reduce_max_sync(0xffffffffu, in ? rec.y : INT_MIN);
+    if ((threadIdx.x & 31) == 0)
+        s_box[threadIdx.x >> 5] = make_int4(x0, x1, y0, y1);
+    __syncthreads();
+    int4 b = s_box[0];
+#pragma unroll
+    for (int q = 1; q < kGridThreads / 32; ++q)
+    {
+        const int4 c = s_box[q];
+        b.x = min(b.x, c.x);
+        b.y = max(b.y, c.y);
+        b.z = min(b.z, c.z);
+        b.w = max(b.w, c.w);
+    }
+    return b;
+}
 
 // Returns, for thread t < m, the key of the t-th visibility of the task in
 // TaskKey order; its low 8 bits are the task-relative index of that
@@ -220,7 +274,7 @@ __device__ __forceinline__ bool same_taps(const TapVis<GT>& a,
 {
     return a.origin == b.origin && a.mu == b.mu && a.mv == b.mv &&
            a.tu == b.tu && a.cp == b.cp && a.cn == b.cn &&
-           a.rowbase == b.rowbase;
+           a.base == b.base;
 }
 
 // Predicated complex flush: one vector reduction when `pred` holds, no
@@ -424,8 +478,11 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
             // The kernel row base of this visibility's column, as a byte
             // address: each tap's address is then one wide multiply-add of
             // its row by the row pitch in bytes.
-            const char* __restrict__ kp = reinterpret_cast<const char*>(
-                slab + (unsigned)(v.rowbase - row_shift + col));
+            const char* __restrict__ kp =
+                (GMEM ? reinterpret_cast<const char*>(v.base)
+                      : reinterpret_cast<const char*>(
+                            slab + ((int)v.base - row_shift))) +
+                (size_t)(unsigned)col * sizeof(KT);
             const unsigned cell0 = v.origin + ru;
             // All of this visibility's kernel values for the thread's rows
             // are requested before any is used.
@@ -538,6 +595,7 @@ romein_grid_kernel(const GridArgs a)
     __shared__ uint32_t s_order[kGridThreads];
     __shared__ int s_run_begin[kMaxOffsets], s_run_end[kMaxOffsets];
     __shared__ unsigned char s_head[kTaskMax];
+    __shared__ int4 s_box[kGridThreads / 32];
     __shared__ int s_warp_heads[kGridThreads / 32];
 
     unsigned long long* status = &a.counters[CNT_STATUS];
@@ -584,7 +642,6 @@ romein_grid_kernel(const GridArgs a)
         }
         // The task's job: its cube, grid and geometry.
         const JobDesc& jd = a.jobs[a.task_job[task]];
-        const TaskKey tk(jd.half, !STAGED);
         const int t = threadIdx.x;
         // Gather the task's visibilities (sorted positions begin .. begin +
         // m - 1) straight from the caller's arrays: record, visibility and
@@ -597,6 +654,7 @@ romein_grid_kernel(const GridArgs a)
                       "raw records fit the tap-record array");
         RawVis<GT>* s_raw = reinterpret_cast<RawVis<GT>*>(s_vis);
         uint32_t key = 0xffffffffu;
+        int4 myrec = make_int4(0, 0, 0, 0);
         if (t < m)
         {
             const uint32_t i = a.order[begin + t];
@@ -614,12 +672,12 @@ romein_grid_kernel(const GridArgs a)
             rv.vis.x = re;
             rv.vis.y = im;
             s_raw[t] = rv;
-            key = tk.make(rv.rec, t);
+            myrec = rv.rec;
         }
-        // Order the task's visibilities by (row offset, cell): each run of
-        // one row offset reads one W-row block of the plane's slab, and
-        // consecutive visibilities are neighbours.  (Its block barriers also
-        // publish the raw records.)
+        const TaskKey tk(jd.half, task_box(t < m, myrec, s_box));
+        if (t < m) key = tk.template make<!STAGED>(myrec, t);
+        // Order the task's visibilities (see TaskKey): consecutive ones are
+        // neighbours.  (Its block barriers also publish the raw records.)
         static_assert(kGridThreads >= 64, "task_order has a block barrier");
         key = task_order(key, s_order);
         const KT* __restrict__ slabs = static_cast<const KT*>(jd.slabs);
@@ -637,7 +695,8 @@ romein_grid_kernel(const GridArgs a)
         const int grid_size = jd.grid_size;
         const int offsets = 2 * jd.half + 1;
         const int plane = r0.z & 0x7fffffff;
-        const PlaneDesc d = static_cast<const PlaneDesc*>(jd.planes)[plane];
+        const PlaneDesc* __restrict__ planes = jd.planes;
+        const PlaneDesc d = planes[plane];
         const int w = 2 * d.support + 1;
         // No kept footprint is wider than its grid; a task that says
         // otherwise is malformed (and its cells could leave the grid).
@@ -656,8 +715,10 @@ romein_grid_kernel(const GridArgs a)
         TapVis<GT> tv;
         if (t < m)
         {
-            tv = derive<GT>(mine.rec, mine.vis, d, grid_size, jd.oversample,
-                            jd.half, status);
+            tv = derive<GT, KT>(mine.rec, mine.vis,
+                                planes[mine.rec.z & 0x7fffffff],
+                                STAGED ? nullptr : slabs, grid_size,
+                                jd.oversample, jd.half, status);
             s_vis[t] = tv;
         }
         __syncthreads();
@@ -709,8 +770,7 @@ romein_grid_kernel(const GridArgs a)
         if (!STAGED)
         {
             dispatch_cpt<GT, KT, COUNT, true>(cpt, s_vis, m, w, d.pitch, 0,
-                                        slabs + d.offset, fl, grid_size,
-                                        flushes);
+                                        slabs, fl, grid_size, flushes);
             continue;
         }
         const unsigned block_elems = (unsigned)w * (unsigned)d.pitch;

@@ -35,6 +35,7 @@ struct PlaneDesc
     int L;              // column positions per oversample phase
     int pitch;          // row length of the slab in elements (os * L)
     int rows;           // slab rows: (2H + 1) * (2S + 1)
+    int group;          // rank of S among the cube's distinct supports
     long long offset;   // element offset of the slab in the slab array
     unsigned bytes;     // slab bytes, rounded up to 16
     float scale;        // stored value = true value / scale (1 unless F16/BF16)
@@ -189,6 +190,7 @@ struct oskar_B200Cube
     unsigned max_slab_bytes = 0;
     unsigned max_block_bytes = 0;   // largest W-row block (one row offset)
     int max_support = 0;
+    std::vector<int> group_support;   // the distinct supports, ascending
     std::vector<b200::PlaneDesc> planes;
     b200::DeviceBuffer d_planes, d_slabs, d_norm_table, d_support;
 };
@@ -228,16 +230,21 @@ int cube_build(oskar_B200Cube* cube, const void* d_conv_func,
 
 // ---- prep.cu / grid_romein.cu ---------------------------------------------
 // Sort key, most significant first:
-//   job | coarse tile (row-major: row, column) | w-plane |
+//   job | coarse tile (row-major: row, column) | group |
 //   cell inside the tile (Morton)
-// with a skip flag above all of them.
+// with a skip flag above all of them.  The group is the rank of the w-plane's
+// support: planes of one support share a footprint width and slab geometry,
+// so one task can hold points of all of them, and neighbours in the order are
+// then much closer than points of a single plane.  (The staged kernel-value
+// path copies one plane's rows at a time; its group is the w-plane.)
 struct KeyLayout
 {
     int coarse_shift;  // log2 of the coarse tile side (cells)
     int coarse_bits;   // bits per axis of the coarse tile index
     int fine_shift;    // cells dropped inside a coarse tile
     int fine_bits;     // bits per axis of the fine index
-    int plane_bits;
+    int group_bits;
+    int by_plane;      // group = w-plane
     int job_bits;
     int job_shift;     // position of the job field
     int total_bits;    // key bits below the skip flag
@@ -245,9 +252,19 @@ struct KeyLayout
 // Layout for the largest grid and plane count of the batch; false if the
 // fields cannot fit 31 bits.
 // tile_shift > 0 sets the coarse tile side to 2^tile_shift cells (at least
-// 64, at most the grid); 0 picks grid_size / 16.
+// 64, at most the grid); 0 picks grid_size / 16.  num_groups: most distinct
+// supports of any job's cube; 0 groups by w-plane.
 bool make_key_layout(int grid_size, int num_planes, int num_jobs,
-                     KeyLayout* out, int tile_shift = 0);
+                     KeyLayout* out, int tile_shift = 0, int num_groups = 0);
+// Sets each plane's group and returns the groups' supports (ascending, at
+// most 128: supports are <= 127).
+std::vector<int> assign_groups(PlaneDesc* planes, int num_planes);
+// Points per task of each group, as powers of two (at most kTaskMax).
+struct TaskSizes
+{
+    uint32_t group_mask;           // of the group field; 0: log2_max[0] for all
+    unsigned char log2_max[128];
+};
 
 // One job of a batch, host side.
 struct HostJob

@@ -80,6 +80,46 @@ double coord_scale_of(double frequency_hz)
     return frequency_hz > 0.0 ? frequency_hz / 299792458.0 : 1.0;
 }
 
+// Points per task by group.  A task's time goes with its taps, 30 times more
+// for the widest footprints than for the narrowest, and the last tasks of a
+// launch leave the device idle: wide groups get smaller tasks, to at most
+// `cap` taps, the smaller the fewer points the launch has to fill the
+// device with.  Smaller tasks merge and share less and repeat their set-up.
+// Gridding time without a cap and with caps of 4e5, 2e5, 1e5, 5e4 taps:
+//   39.2 M points on 8192^2    16.28, 16.29, 16.55, 17.35, 18.92 ms
+//   2.2 M points on 3000^2      551, 553, 525, 519, 557 us
+//   0.24 M points on 1024^2      49, 51, 47, 46, 53 us
+//   the drop-in's bands (1.3 M host points on 2048^2, whole call)
+//                              2.58, 2.62, 2.54, 2.33, 2.37 ms
+static TaskSizes task_sizes(const KeyLayout& kl, int num_jobs,
+                            const HostJob* jobs, size_t points)
+{
+    TaskSizes t{};
+    int full = 0;
+    while ((1 << full) < kTaskMax) ++full;
+    if (kl.by_plane)
+    {
+        t.log2_max[0] = (unsigned char)full;
+        return t;
+    }
+    const long long cap = points < (size_t(1) << 18) ? 100000
+                          : points < (size_t(1) << 23) ? 200000 : 400000;
+    t.group_mask = (1u << kl.group_bits) - 1u;
+    memset(t.log2_max, full, sizeof(t.log2_max));
+    for (int j = 0; j < num_jobs; ++j)
+    {
+        const std::vector<int>& support = jobs[j].cube->group_support;
+        for (size_t g = 0; g < support.size(); ++g)
+        {
+            const long long w = 2ll * support[g] + 1;
+            int l = full;
+            while (l > 5 && ((w * w) << l) > cap) --l;
+            t.log2_max[g] = std::min(t.log2_max[g], (unsigned char)l);
+        }
+    }
+    return t;
+}
+
 int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
               int num_jobs, const HostJob* jobs, cudaStream_t st,
               bool degrid, BandPlan* bands, int time_slices)
@@ -105,7 +145,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
 
     // Job table (host, pinned: it is the source of an async upload).
     size_t n = 0, max_points = 0, comp_floats = 0;
-    int max_grid = 1, max_planes = 1;
+    int max_grid = 1, max_planes = 1, max_groups = 1;
     unsigned max_block = 0;
     for (int j = 0; j < num_jobs; ++j)
     {
@@ -113,6 +153,8 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         max_points = std::max(max_points, jobs[j].num_points);
         max_grid = std::max(max_grid, jobs[j].grid_size);
         max_planes = std::max(max_planes, jobs[j].cube->num_planes);
+        max_groups = std::max(max_groups,
+                              (int)jobs[j].cube->group_support.size());
         max_block = std::max(max_block, jobs[j].cube->max_block_bytes);
         if (comp)
             comp_floats += 2 * (size_t)jobs[j].grid_size * jobs[j].grid_size;
@@ -123,7 +165,16 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     // Launch shape: the options', else the workspace's tuned one.
     const int tile_shift = opt->tile_shift > 0 ? opt->tile_shift
                            : ws->tuned_launch ? ws->tuned_tile_shift : 0;
-    if (!make_key_layout(max_grid, max_planes, num_jobs, &kl, tile_shift))
+    // Kernel values are read through L1 unless staging is asked for: on
+    // plain_large the L1 path is as fast as staging each row-offset run's
+    // W-row block into shared memory (24.2 ms vs 24.8 ms with FP16 slabs,
+    // 30.2 ms with FP32 slabs, whose blocks cap residency at 2 CTAs/SM).
+    const bool staged = !degrid &&
+                        (opt->staging == 1 ||
+                         (opt->staging == 0 && !comp && ws->tuned_launch &&
+                          ws->tuned_staging == 1));
+    if (!make_key_layout(max_grid, max_planes, num_jobs, &kl, tile_shift,
+                         staged || comp ? 0 : max_groups))
         return OSKAR_B200_ERR_UNSUPPORTED;
     if (bands)
     {
@@ -339,8 +390,10 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
                                  cudaMemcpyDeviceToHost, st));
         return OSKAR_B200_OK;
     }
+    const TaskSizes sizes = task_sizes(
+        kl, num_jobs, jobs, bands ? n / bands->num_bands : n);
     B200_TRY(launch_tasks(keys[which], n, counters, 2 * kl.fine_bits,
-                          kl.job_shift, kTaskMax,
+                          kl.job_shift, sizes,
                           static_cast<uint32_t*>(ws->flags.ptr),
                           ws->scan_tmp.ptr,
                           static_cast<uint32_t*>(ws->task_start.ptr),
@@ -366,13 +419,6 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         memcpy(ga.cpt, ws->tune, sizeof(ga.cpt));
     else
         default_tune_table(ga.cpt);
-    // Kernel values are read through L1 unless staging is asked for: on
-    // plain_large the L1 path is as fast as staging each row-offset run's
-    // W-row block into shared memory (24.2 ms vs 24.8 ms with FP16 slabs,
-    // 30.2 ms with FP32 slabs, whose blocks cap residency at 2 CTAs/SM).
-    const bool staged = opt->staging == 1 ||
-                        (opt->staging == 0 && !comp && ws->tuned_launch &&
-                         ws->tuned_staging == 1);
     if (staged && grid_smem_bytes(dbl, max_block, true) > ws->smem_optin)
         return OSKAR_B200_ERR_UNSUPPORTED;
     if (comp)

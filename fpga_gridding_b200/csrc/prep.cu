@@ -4,6 +4,7 @@
 // norms and the plane histograms; then, after the sort, the gridding work
 // list (tasks).
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
 #include "internal.h"
@@ -16,8 +17,21 @@ namespace b200 {
 // (three 8-bit passes) gave sort 2.17 -> 1.47 ms, gridding 20.3 -> 22.2 ms.
 constexpr int kKeyBits = 32;
 
+std::vector<int> assign_groups(PlaneDesc* planes, int num_planes)
+{
+    std::vector<int> s((size_t)num_planes);
+    for (int p = 0; p < num_planes; ++p) s[p] = planes[p].support;
+    std::sort(s.begin(), s.end());
+    s.erase(std::unique(s.begin(), s.end()), s.end());
+    for (int p = 0; p < num_planes; ++p)
+        planes[p].group = (int)(std::lower_bound(s.begin(), s.end(),
+                                                 planes[p].support) -
+                                s.begin());
+    return s;
+}
+
 bool make_key_layout(int grid_size, int num_planes, int num_jobs,
-                     KeyLayout* out, int tile_shift)
+                     KeyLayout* out, int tile_shift, int num_groups)
 {
     KeyLayout k{};
     int gbits = 0;
@@ -30,18 +44,23 @@ bool make_key_layout(int grid_size, int num_planes, int num_jobs,
         k.coarse_shift = std::max(6, std::min(tile_shift, std::max(gbits, 6)));
     const int ctiles = (grid_size + (1 << k.coarse_shift) - 1) >> k.coarse_shift;
     while ((1 << k.coarse_bits) < ctiles) ++k.coarse_bits;
-    while ((1 << k.plane_bits) < num_planes) ++k.plane_bits;
+    int plane_bits = 0;
+    while ((1 << plane_bits) < num_planes) ++plane_bits;
+    k.by_plane = num_groups == 0;
+    if (k.by_plane) num_groups = num_planes;
+    while ((1 << k.group_bits) < num_groups) ++k.group_bits;
     while ((1 << k.job_bits) < num_jobs) ++k.job_bits;
     k.fine_shift = 0;
     k.fine_bits = k.coarse_shift;
-    const int fixed = k.job_bits + 2 * k.coarse_bits + k.plane_bits + 1;
-    if (fixed > 32) return false;
+    // (The same jobs are refused whatever the grouping.)
+    if (k.job_bits + 2 * k.coarse_bits + plane_bits + 1 > 32) return false;
+    const int fixed = k.job_bits + 2 * k.coarse_bits + k.group_bits + 1;
     while (fixed + 2 * k.fine_bits > kKeyBits && k.fine_bits > 0)
     {
         ++k.fine_shift;
         --k.fine_bits;
     }
-    k.job_shift = 2 * k.coarse_bits + k.plane_bits + 2 * k.fine_bits;
+    k.job_shift = 2 * k.coarse_bits + k.group_bits + 2 * k.fine_bits;
     k.total_bits = k.job_shift + k.job_bits;
     *out = k;
     return true;
@@ -73,7 +92,7 @@ __device__ __forceinline__ uint32_t spread_bits(uint32_t x)
 }
 
 __device__ __forceinline__ uint32_t make_key(const KeyLayout& k, int job,
-                                             int gu, int gv, int plane)
+                                             int gu, int gv, int group)
 {
     const uint32_t cu = (uint32_t)gu >> k.coarse_shift;
     const uint32_t cv = (uint32_t)gv >> k.coarse_shift;
@@ -86,8 +105,8 @@ __device__ __forceinline__ uint32_t make_key(const KeyLayout& k, int job,
     const uint32_t coarse = (cv << k.coarse_bits) | cu;
     const uint32_t fine = spread_bits(fu) | (spread_bits(fv) << 1);
     return ((uint32_t)job << k.job_shift) |
-           (coarse << (k.plane_bits + 2 * k.fine_bits)) |
-           ((uint32_t)plane << (2 * k.fine_bits)) | fine;
+           (coarse << (k.group_bits + 2 * k.fine_bits)) |
+           ((uint32_t)group << (2 * k.fine_bits)) | fine;
 }
 
 __device__ __forceinline__ PlaceConsts place_consts(const JobDesc& jd)
@@ -152,7 +171,9 @@ prep_kernel(const PrepArgs a)
                 a.rec[g] = make_int4(p.gu, p.gv,
                                      p.plane | (p.conj < 0 ? (int)0x80000000 : 0),
                                      (p.off_u + half) | ((p.off_v + half) << 16));
-                a.keys[g] = make_key(a.key, job, p.gu, p.gv, p.plane);
+                a.keys[g] = make_key(a.key, job, p.gu, p.gv,
+                                     a.key.by_plane
+                                         ? p.plane : jd.planes[p.plane].group);
                 double s = jd.norm_table[((size_t)p.plane * span +
                                           (p.off_v + half)) * span +
                                          (p.off_u + half)];
@@ -250,31 +271,33 @@ __global__ void finalize_prep_kernel(const PrepArgs a)
 // Task list in two passes over the sorted keys, tiles of kTaskTile
 // positions: each tile counts its task starts, the tile counts are scanned,
 // and each tile writes its starts at its offset.  A task starts at sorted
-// position s < valid when s == 0, s % task_max == 0, or the key above the
-// fine cell bits changes.
+// position s < valid when s == 0, at every multiple of its group's task size,
+// or where the key above the fine cell bits changes.
 constexpr int kTaskTile = 4096;
 constexpr int kTaskThreads = 256;
 
 __device__ __forceinline__ bool task_starts_at(const uint32_t* keys, size_t s,
                                                size_t valid, int fine_bits,
-                                               int task_max)
+                                               const TaskSizes& sizes)
 {
     return s < valid &&
-           (s == 0 || s % (size_t)task_max == 0 ||
+           (s == 0 ||
+            (s & ((1u << sizes.log2_max[(keys[s] >> fine_bits) &
+                                        sizes.group_mask]) - 1u)) == 0 ||
             (keys[s] >> fine_bits) != (keys[s - 1] >> fine_bits));
 }
 
 __global__ void __launch_bounds__(kTaskThreads)
 task_count_kernel(const uint32_t* __restrict__ keys, size_t n,
                   const unsigned long long* __restrict__ counters,
-                  int fine_key_bits, int task_max,
+                  int fine_key_bits, const TaskSizes sizes,
                   uint32_t* __restrict__ tile_counts)
 {
     const size_t valid = n - counters[CNT_SKIPPED];
     const size_t tile0 = (size_t)blockIdx.x * kTaskTile;
     unsigned c = 0;
     for (int k = threadIdx.x; k < kTaskTile; k += kTaskThreads)
-        c += task_starts_at(keys, tile0 + k, valid, fine_key_bits, task_max);
+        c += task_starts_at(keys, tile0 + k, valid, fine_key_bits, sizes);
     c = warp_sum(c);
     __shared__ unsigned s_w[kTaskThreads / 32];
     if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = c;
@@ -292,7 +315,7 @@ task_count_kernel(const uint32_t* __restrict__ keys, size_t n,
 __global__ void __launch_bounds__(kTaskThreads)
 task_write_kernel(const uint32_t* __restrict__ keys, size_t n,
                   unsigned long long* __restrict__ counters,
-                  int fine_key_bits, int task_max, int job_shift,
+                  int fine_key_bits, const TaskSizes sizes, int job_shift,
                   const uint32_t* __restrict__ tile_counts,
                   const uint32_t* __restrict__ tile_offsets,
                   uint32_t* __restrict__ task_start,
@@ -307,8 +330,7 @@ task_write_kernel(const uint32_t* __restrict__ keys, size_t n,
     for (int r = 0; r < kTaskTile; r += kTaskThreads)
     {
         const size_t pos = tile0 + r + threadIdx.x;
-        const bool f = task_starts_at(keys, pos, valid, fine_key_bits,
-                                      task_max);
+        const bool f = task_starts_at(keys, pos, valid, fine_key_bits, sizes);
         const unsigned ball = __ballot_sync(0xffffffffu, f);
         if (lane == 0) s_w[warp] = __popc(ball);
         __syncthreads();
@@ -393,21 +415,21 @@ size_t task_tiles(size_t n) { return (n + kTaskTile - 1) / kTaskTile; }
 
 cudaError_t launch_tasks(const uint32_t* sorted_keys, size_t n,
                          unsigned long long* counters, int fine_key_bits,
-                         int job_shift, int task_max, uint32_t* tile_counts,
-                         void* scan_tmp, uint32_t* task_start,
+                         int job_shift, const TaskSizes& sizes,
+                         uint32_t* tile_counts, void* scan_tmp, uint32_t* task_start,
                          uint32_t* task_job, cudaStream_t st, int* launches)
 {
     const size_t tiles = task_tiles(n);
     if (tiles == 0) return cudaSuccess;
     uint32_t* tile_offsets = tile_counts + tiles;
     task_count_kernel<<<(unsigned)tiles, kTaskThreads, 0, st>>>(
-        sorted_keys, n, counters, fine_key_bits, task_max, tile_counts);
+        sorted_keys, n, counters, fine_key_bits, sizes, tile_counts);
     cudaError_t e = exclusive_scan_u32(tile_counts, tile_offsets, tiles,
                                        scan_tmp, st, launches);
     if (e != cudaSuccess) return e;
     if (launches) *launches += 2;
     task_write_kernel<<<(unsigned)tiles, kTaskThreads, 0, st>>>(
-        sorted_keys, n, counters, fine_key_bits, task_max, job_shift,
+        sorted_keys, n, counters, fine_key_bits, sizes, job_shift,
         tile_counts, tile_offsets, task_start, task_job);
     return cudaGetLastError();
 }
@@ -455,7 +477,7 @@ cudaError_t launch_band_first(const uint32_t* sorted_keys,
                               uint32_t* band_first, int num_sms,
                               cudaStream_t st)
 {
-    const int shift = kl.plane_bits + 2 * kl.fine_bits + kl.coarse_bits;
+    const int shift = kl.group_bits + 2 * kl.fine_bits + kl.coarse_bits;
     const uint32_t mask = (1u << kl.coarse_bits) - 1u;
     const unsigned blocks = grid_blocks(n + 1, num_sms, 8, 256);
     band_first_kernel<<<blocks, 256, 0, st>>>(sorted_keys, task_start,

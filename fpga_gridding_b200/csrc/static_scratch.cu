@@ -32,7 +32,7 @@ namespace b200 {
 
 size_t static_cube_geometry(int num_planes, const int* support,
                             int oversample, std::vector<PlaneDesc>* planes,
-                            unsigned* max_block_bytes);
+                            unsigned* max_block_bytes, int* num_groups);
 int static_cube_fill(const float* d_conv, int num_planes, int oversample,
                      int conv_size_half, const PlaneDesc* d_planes,
                      float2* d_slabs, double* d_norm_table, cudaStream_t st);
@@ -123,13 +123,15 @@ extern "C" int oskar_b200_grid_f_static(
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device);
     if (major != 10) return OSKAR_B200_ERR_NO_DEVICE;
     KeyLayout kl;
-    if (!make_key_layout(grid_size, P, 1, &kl)) return OSKAR_B200_ERR_UNSUPPORTED;
-
     // Carve the scratch; refuse jobs that do not fit.
     std::vector<PlaneDesc> planes;
     unsigned max_block = 0;
+    int groups = 0;
     const size_t slab_bytes = static_cube_geometry(P, support, oversample,
-                                                   &planes, &max_block);
+                                                   &planes, &max_block,
+                                                   &groups);
+    if (!make_key_layout(grid_size, P, 1, &kl, 0, groups))
+        return OSKAR_B200_ERR_UNSUPPORTED;
     const size_t n = num_points;
     const int bpj = prep_blocks_per_job(n, 1, num_sms);
     const int span = 2 * half + 1;
@@ -232,8 +234,10 @@ extern "C" int oskar_b200_grid_f_static(
     int which = 0;
     B200_S(radix_sort_pairs(keys, vals, n, kl.total_bits + 1, scan_tmp, s,
                             &which, nullptr));
+    TaskSizes sizes{};
+    while ((1 << sizes.log2_max[0]) < kTaskMax) ++sizes.log2_max[0];
     B200_S(launch_tasks(keys[which], n, counters, 2 * kl.fine_bits,
-                        kl.job_shift, kTaskMax, tile_counts, scan_tmp,
+                        kl.job_shift, sizes, tile_counts, scan_tmp,
                         task_start, task_job, s, nullptr));
     GridArgs ga{};
     ga.order = vals[which];
