@@ -45,6 +45,12 @@ __device__ __forceinline__ void red_add_c(double* addr, double re, double im)
                  :: "l"(addr + 1), "d"(im) : "memory");
 }
 
+__device__ __forceinline__ void red_add(double* addr, double x)
+{
+    asm volatile("red.relaxed.gpu.global.add.f64 [%0], %1;"
+                 :: "l"(addr), "d"(x) : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // mbarrier and bulk (non-tensor) TMA copies into this CTA's shared memory.
 // ---------------------------------------------------------------------------

@@ -86,6 +86,16 @@ __device__ __forceinline__ void cmac(double2& acc, const double2 c0,
     acc.y = fma(c1.y, k.y, acc.y);
 }
 
+// FP32 terms onto FP64 sums: each tap's two products are rounded to FP32
+// (relative error 2^-23 of the tap, no larger than an FP32 running sum's
+// rounding), their sum over the taps is not.
+__device__ __forceinline__ void cmac(double2& acc, const float2 c0,
+                                     const float2 c1, const float2 k)
+{
+    acc.x += (double)fmaf(c1.x, k.y, c0.x * k.x);
+    acc.y += (double)fmaf(c1.y, k.y, c0.y * k.x);
+}
+
 // slabs: the cube's slab array (L1 path), or null (staged path).
 template <typename GT, typename KT>
 __device__ __forceinline__ TapVis<GT> derive(const int4 rec,
@@ -336,13 +346,20 @@ __device__ __forceinline__ TaskLayout task_layout(int w)
 }
 
 // Grid flush policies.  PlainFlush: one predicated vector reduction.
-// CompensatedFlush (FP32): the addition returns the old value; Knuth's
-// TwoSum recovers the exact rounding error of old + x (the atomic rounds to
-// nearest even), which is added to a compensation grid folded into the grid
-// at the end of the job.  Its branch is taken only when the lane flushes.
+// CompensatedFlush (FP32 grids): the running sums are FP64 and go to FP64
+// planes of sums, one of the real and one of the imaginary parts, which are
+// added to the grid at the end of the job.  Every cell is then rounded to FP32
+// once.  Two fire-and-forget reductions of consecutive lanes replace the
+// returning FP32 atomic whose rounding error (Knuth's TwoSum) was collected in
+// an error grid: 3.4 M points on 4096^2, oversample 8, gridding 10.6 ->
+// 5.1 ms, error against FP64 5.3e-8 -> 3.3e-8 (FP32 running sums with these
+// reductions: 8e-8; 3 CTAs per SM instead of 4: 5.2 ms).  The sums take 16
+// bytes per cell, the error grid took 8: where that much does not fit, the
+// tasks run twice with one plane of sums (see pipeline.cu).
 template <typename GT>
 struct PlainFlush
 {
+    using Acc = typename Vec2<GT>::type;
     GT* grid;
     // FP32: the compare, the predicated reduction and the reset of the
     // running sum in one block of PTX.  When `valid` and cell != cur, the
@@ -369,35 +386,26 @@ struct PlainFlush
     }
 };
 
-__device__ __forceinline__ float two_sum_err(float a, float b)
-{
-    const float s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    return __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-}
-
 struct CompensatedFlush
 {
+    using Acc = double2;
     float* grid;
-    float* comp;
+    double* re;    // sums of this pass, or null
+    double* im;
     bool active;   // false: this task's cells are not compensated
     __device__ __forceinline__ void operator()(bool pred, unsigned cell,
-                                               float re, float im) const
+                                               double x, double y) const
     {
-        if (!active)
-        {
-            red_add_c_if(pred, grid + 2 * (size_t)cell, re, im);
-            return;
-        }
         if (!pred) return;
-        float ore, oim;
-        asm volatile("atom.relaxed.gpu.global.add.v2.f32 {%0, %1}, [%2], {%3, %4};"
-                     : "=f"(ore), "=f"(oim)
-                     : "l"(grid + 2 * (size_t)cell), "f"(re), "f"(im)
-                     : "memory");
-        const float er = two_sum_err(ore, re), ei = two_sum_err(oim, im);
-        if (er != 0.f || ei != 0.f)
-            red_add_c(comp + 2 * (size_t)cell, er, ei);
+        if (active)
+        {
+            if (re) red_add(re + cell, x);
+            if (im) red_add(im + cell, y);
+        }
+        else if (re)
+        {
+            red_add_c(grid + 2 * (size_t)cell, (float)x, (float)y);
+        }
     }
 };
 
@@ -446,7 +454,8 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
         // Every slot runs the same straight-line code (a per-slot `break`
         // cost a branch and convergence barriers per tap: 19.9 -> 16.8 ms
         // at plain_large without it); masked slots never flush.
-        typename Vec2<GT>::type acc[CPT];   // (re, im) of each row's cell
+        using Acc = typename FL::Acc;
+        Acc acc[CPT];                       // (re, im) of each row's cell
         unsigned cur[CPT];
         constexpr bool kFused =
             std::is_same<FL, PlainFlush<float>>::value && !COUNT;
@@ -461,7 +470,7 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
             {
                 const unsigned rv = min(xb + q, xb + q - (unsigned)w);
                 cur[q] = v.origin + ru + rv * (unsigned)grid_size;
-                acc[q].x = acc[q].y = GT(0);
+                acc[q].x = acc[q].y = 0;
             }
         }
         // Two visibilities per iteration: the running cells then alternate
@@ -510,8 +519,8 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
                     const bool change = q >= skip && cell != cur[q];
                     flush(change, cur[q], acc[q].x, acc[q].y);
                     if (COUNT) flushes += change;
-                    acc[q].x = change ? GT(0) : acc[q].x;
-                    acc[q].y = change ? GT(0) : acc[q].y;
+                    acc[q].x = change ? 0 : acc[q].x;
+                    acc[q].y = change ? 0 : acc[q].y;
                 }
                 cur[q] = cell;
                 typename Vec2<GT>::type kk;
@@ -557,23 +566,14 @@ template <> struct FlushFor<float, true> { using type = CompensatedFlush; };
 
 template <typename GT, bool COMP>
 __device__ __forceinline__ typename FlushFor<GT, COMP>::type
-make_flush(void* grid, void* comp, bool active);
-template <>
-__device__ __forceinline__ PlainFlush<float> make_flush<float, false>(void* grid, void*, bool)
+make_flush(const JobDesc& jd, int comp_part, bool active)
 {
-    return PlainFlush<float>{static_cast<float*>(grid)};
-}
-template <>
-__device__ __forceinline__ PlainFlush<double> make_flush<double, false>(void* grid, void*, bool)
-{
-    return PlainFlush<double>{static_cast<double*>(grid)};
-}
-template <>
-__device__ __forceinline__ CompensatedFlush make_flush<float, true>(void* grid, void* comp,
-                                                                    bool active)
-{
-    return CompensatedFlush{static_cast<float*>(grid), static_cast<float*>(comp),
-                            active};
+    if constexpr (COMP)
+        return CompensatedFlush{static_cast<float*>(jd.grid),
+                                comp_part ? nullptr : jd.comp[0],
+                                jd.comp[comp_part ? 0 : 1], active};
+    else
+        return PlainFlush<GT>{static_cast<GT*>(jd.grid)};
 }
 
 // At least grid_ctas_per_sm<GT>() CTAs per SM.  FP32: with the
@@ -691,7 +691,7 @@ romein_grid_kernel(const GridArgs a)
             comp_here = abs(r0.x - c) <= a.comp_radius &&
                         abs(r0.y - c) <= a.comp_radius;
         }
-        const auto fl = make_flush<GT, COMP>(jd.grid, jd.comp, comp_here);
+        const auto fl = make_flush<GT, COMP>(jd, a.comp_part, comp_here);
         const int grid_size = jd.grid_size;
         const int offsets = 2 * jd.half + 1;
         const int plane = r0.z & 0x7fffffff;
@@ -913,37 +913,31 @@ void default_tune_table(unsigned char* cpt)
 
 namespace {
 
-// Block (x, j) folds part of job j's error grid into its grid.
-__global__ void fold_kernel(const JobDesc* __restrict__ jobs)
+// Block (x, j) adds part of job j's FP64 sums to its grid (jobs of a batch
+// may share a grid: a reduction per cell).
+__global__ void fold_kernel(const JobDesc* __restrict__ jobs, int comp_part)
 {
     const JobDesc& jd = jobs[blockIdx.y];
-    if (!jd.comp) return;
-    float2* grid = static_cast<float2*>(jd.grid);
-    float2* comp = static_cast<float2*>(jd.comp);
+    const double* re = comp_part ? nullptr : jd.comp[0];
+    const double* im = jd.comp[comp_part ? 0 : 1];
+    float* grid = static_cast<float*>(jd.grid);
     const size_t cells = (size_t)jd.grid_size * (size_t)jd.grid_size;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cells;
          i += (size_t)gridDim.x * blockDim.x)
     {
-        const float2 c = comp[i];
-        if (c.x != 0.f || c.y != 0.f)
-        {
-            float2 g = grid[i];
-            g.x += c.x;
-            g.y += c.y;
-            grid[i] = g;
-            comp[i] = make_float2(0.f, 0.f);
-        }
+        const float x = re ? (float)re[i] : 0.f, y = im ? (float)im[i] : 0.f;
+        if (x != 0.f || y != 0.f) red_add_c(grid + 2 * i, x, y);
     }
 }
 
 }  // namespace
 
-cudaError_t launch_fold_jobs(const JobDesc* jobs, int num_jobs, int num_sms,
-                             cudaStream_t st)
+cudaError_t launch_fold_jobs(const JobDesc* jobs, int num_jobs, int comp_part,
+                             int num_sms, cudaStream_t st)
 {
     int bx = num_sms * 8 / (num_jobs > 0 ? num_jobs : 1);
     if (bx < 4) bx = 4;
-    fold_kernel<<<dim3(bx, num_jobs), 256, 0, st>>>(jobs);
+    fold_kernel<<<dim3(bx, num_jobs), 256, 0, st>>>(jobs, comp_part);
     return cudaGetLastError();
 }
 

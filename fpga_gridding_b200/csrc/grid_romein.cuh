@@ -27,6 +27,8 @@ struct GridArgs
     unsigned long long* counters;
     unsigned block_smem_bytes;  // set by launch_grid
     int comp_radius;            // see oskar_B200Options::compensate_radius
+    int comp_part;              // 0: first pass over the tasks; 1: the second,
+                                // for the imaginary sums alone
     int count_flushes;          // count grid atomics (statistics)
     unsigned char cpt[kTuneMax];
     // Optional task range [range[0], range[1]) with its own work-queue
@@ -43,8 +45,8 @@ cudaError_t launch_grid(const GridArgs& a, int data_is_double,
                         int kernel_type, unsigned max_block_bytes, bool staged,
                         bool compensated, int num_sms, cudaStream_t st,
                         int* ctas_out);
-// For every job with an error grid: grid += comp, comp = 0.
-cudaError_t launch_fold_jobs(const JobDesc* jobs, int num_jobs, int num_sms,
-                             cudaStream_t st);
+// For every job with FP64 sums: grid += the sums.
+cudaError_t launch_fold_jobs(const JobDesc* jobs, int num_jobs, int comp_part,
+                             int num_sms, cudaStream_t st);
 
 }  // namespace b200

@@ -51,7 +51,8 @@ struct JobDesc
     const void* vis;
     const void* weight;
     void* grid;
-    void* comp;                   // error grid (ACCUM_COMPENSATED) or null
+    double* comp[2];              // FP64 sums of the real and the imaginary
+                                  // parts (ACCUM_COMPENSATED), each or null
     const PlaneDesc* planes;
     const void* slabs;
     const double* norm_table;
@@ -141,7 +142,7 @@ struct oskar_B200Workspace
     // drop-in staging of the caller's host arrays
     b200::DeviceBuffer in_uu, in_vv, in_ww, in_vis, in_weight, in_grid,
         in_cube, in_norm;
-    // error grid of ACCUM_COMPENSATED
+    // FP64 sums of ACCUM_COMPENSATED
     b200::DeviceBuffer comp_grid;
     // drop-in pipelined upload: copy stream, its events (cube, one per
     // chunk) and the zeroed grid the chunks accumulate into

@@ -144,7 +144,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     };
 
     // Job table (host, pinned: it is the source of an async upload).
-    size_t n = 0, max_points = 0, comp_floats = 0;
+    size_t n = 0, max_points = 0, comp_cells = 0;
     int max_grid = 1, max_planes = 1, max_groups = 1;
     unsigned max_block = 0;
     for (int j = 0; j < num_jobs; ++j)
@@ -157,7 +157,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
                               (int)jobs[j].cube->group_support.size());
         max_block = std::max(max_block, jobs[j].cube->max_block_bytes);
         if (comp)
-            comp_floats += 2 * (size_t)jobs[j].grid_size * jobs[j].grid_size;
+            comp_cells += (size_t)jobs[j].grid_size * jobs[j].grid_size;
     }
     if (n >= 0xffffffffull) return OSKAR_B200_ERR_INVALID_ARGUMENT;
     ws->last_points = n;
@@ -174,7 +174,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
                          (opt->staging == 0 && !comp && ws->tuned_launch &&
                           ws->tuned_staging == 1));
     if (!make_key_layout(max_grid, max_planes, num_jobs, &kl, tile_shift,
-                         staged || comp ? 0 : max_groups))
+                         staged ? 0 : max_groups))
         return OSKAR_B200_ERR_UNSUPPORTED;
     if (bands)
     {
@@ -234,7 +234,15 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     if (ws->jobs_event_pending[slot] && !capturing)
         B200_TRY(cudaEventSynchronize(ws->jobs_event[slot]));
     ws->jobs_event_pending[slot] = 0;
-    if (comp) B200_TRY(ws->comp_grid.ensure(comp_floats * sizeof(float)));
+    // FP64 sums of the real and of the imaginary parts.  Where there is no
+    // room for both, the tasks run twice and share one plane of sums.
+    int comp_passes = comp ? 1 : 0;
+    if (comp && ws->comp_grid.ensure(2 * comp_cells * sizeof(double)) !=
+                    cudaSuccess)
+    {
+        comp_passes = 2;
+        B200_TRY(ws->comp_grid.ensure(comp_cells * sizeof(double)));
+    }
     JobDesc* hj = static_cast<JobDesc*>(ws->h_jobs[slot]);
     size_t first = 0, comp_off = 0;
     for (int j = 0; j < num_jobs; ++j)
@@ -248,8 +256,11 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         d.vis = h.vis;
         d.weight = h.weight;
         d.grid = h.grid;
-        d.comp = comp ? static_cast<float*>(ws->comp_grid.ptr) + comp_off
-                      : nullptr;
+        if (comp)
+        {
+            d.comp[0] = static_cast<double*>(ws->comp_grid.ptr) + comp_off;
+            d.comp[1] = comp_passes == 1 ? d.comp[0] + comp_cells : nullptr;
+        }
         d.planes = static_cast<const PlaneDesc*>(c->d_planes.ptr);
         d.slabs = c->d_slabs.ptr;
         d.norm_table = static_cast<const double*>(c->d_norm_table.ptr);
@@ -272,7 +283,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         d.half = c->half;
         hj[j] = d;
         first += h.num_points;
-        if (comp) comp_off += 2 * (size_t)h.grid_size * h.grid_size;
+        comp_off += (size_t)h.grid_size * h.grid_size;
     }
     const int bpj = prep_blocks_per_job(max_points, num_jobs, ws->num_sms);
     B200_TRY(ws->counters.ensure(sizeof(unsigned long long) * CNT_COUNT));
@@ -421,10 +432,25 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         default_tune_table(ga.cpt);
     if (staged && grid_smem_bytes(dbl, max_block, true) > ws->smem_optin)
         return OSKAR_B200_ERR_UNSUPPORTED;
-    if (comp)
-        B200_TRY(cudaMemsetAsync(ws->comp_grid.ptr, 0,
-                                 comp_floats * sizeof(float), st));
     int ctas = 0;
+    // A pass over the tasks with compensation: its sums start from zero and
+    // are added to the grids at its end.
+    auto begin_pass = [&](int pass) -> cudaError_t {
+        if (!comp) return cudaSuccess;
+        ga.comp_part = pass;
+        cudaError_t e = cudaMemsetAsync(
+            ws->comp_grid.ptr, 0,
+            (comp_passes == 1 ? 2 : 1) * comp_cells * sizeof(double), st);
+        if (e == cudaSuccess && pass)
+            e = cudaMemsetAsync(counters + CNT_TASK_NEXT, 0,
+                                sizeof(unsigned long long), st);
+        return e;
+    };
+    auto end_pass = [&](int pass) -> cudaError_t {
+        if (!comp) return cudaSuccess;
+        launches += 1;
+        return launch_fold_jobs(d_jobs, num_jobs, pass, ws->num_sms, st);
+    };
     if (bands)
     {
         uint32_t* band_first = static_cast<uint32_t*>(ws->bands.ptr);
@@ -457,30 +483,35 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         uint32_t* first = static_cast<uint32_t*>(ws->bands.ptr);
         unsigned long long* queues = reinterpret_cast<unsigned long long*>(
             static_cast<unsigned char*>(ws->bands.ptr) + 128);
-        B200_TRY(launch_slice_bounds(counters, time_slices, first, queues,
-                                     st));
-        launches += 1;
         B200_TRY(mark(3));
-        for (int k = 0; k < time_slices; ++k)
+        for (int pass = 0; pass < std::max(comp_passes, 1); ++pass)
         {
-            ga.range = first + k;
-            ga.queue = queues + k;
-            B200_TRY(launch_grid(ga, dbl, c0->kernel_type, max_block, staged,
-                                 comp, ws->num_sms, st, &ctas));
+            B200_TRY(begin_pass(pass));
+            B200_TRY(launch_slice_bounds(counters, time_slices, first, queues,
+                                         st));
             launches += 1;
+            for (int k = 0; k < time_slices; ++k)
+            {
+                ga.range = first + k;
+                ga.queue = queues + k;
+                B200_TRY(launch_grid(ga, dbl, c0->kernel_type, max_block,
+                                     staged, comp, ws->num_sms, st, &ctas));
+                launches += 1;
+            }
+            B200_TRY(end_pass(pass));
         }
     }
     else
     {
         B200_TRY(mark(3));
-        B200_TRY(launch_grid(ga, dbl, c0->kernel_type, max_block, staged,
-                             comp, ws->num_sms, st, &ctas));
-        launches += 1;
-    }
-    if (comp)
-    {
-        B200_TRY(launch_fold_jobs(d_jobs, num_jobs, ws->num_sms, st));
-        launches += 1;
+        for (int pass = 0; pass < std::max(comp_passes, 1); ++pass)
+        {
+            B200_TRY(begin_pass(pass));
+            B200_TRY(launch_grid(ga, dbl, c0->kernel_type, max_block, staged,
+                                 comp, ws->num_sms, st, &ctas));
+            launches += 1;
+            B200_TRY(end_pass(pass));
+        }
     }
     B200_TRY(mark(4));
     ws->events_recorded = timing ? 1 : 0;

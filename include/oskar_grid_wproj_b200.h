@@ -213,14 +213,14 @@ enum
     OSKAR_B200_KERNEL_BF16 = 2     /* BF16 with a per-plane scale */
 };
 
-/* Grid accumulation for FP32 data.  COMPENSATED: every grid atomic returns
- * the old value, the exact rounding error of the addition (TwoSum) goes to
- * an FP32 error grid in the workspace (grid_size^2 complex), and the error
- * grid is added into the grid at the end of the call. */
+/* Grid accumulation for FP32 data.  COMPENSATED: the job's contributions are
+ * summed in FP64 (two planes of grid_size^2 doubles in the workspace; one
+ * plane and two runs over the points where both do not fit) and added to the
+ * grid once, at the end. */
 enum
 {
     OSKAR_B200_ACCUM_PLAIN = 0,        /* FP32 register sums, FP32 atomics */
-    OSKAR_B200_ACCUM_COMPENSATED = 1   /* plus the compensated grid atomics */
+    OSKAR_B200_ACCUM_COMPENSATED = 1   /* FP64 sums, one rounding per cell */
 };
 
 typedef struct oskar_B200Options

@@ -78,3 +78,46 @@ def test_groups_match_oracle(oracle, name, oversample, spread, single, accum):
         abs(n1), float(np.abs(ref["conv_func"]).max()) * w["uu"].size * 100)
     cube.close()
     ws.close()
+
+
+def test_compensated_with_one_plane_of_sums(oracle):
+    """No memory for both planes of FP64 sums (the allocation is made to
+    fail): the job runs twice with one plane and gives the same result, with
+    compensation everywhere and within a radius."""
+    w = _job("mixed", 4, 100.0)
+    ref = dict(w)
+    for k in ("conv_func", "uu", "vv", "ww", "vis", "weight"):
+        ref[k] = np.asarray(w[k], np.float32).astype(np.float64)
+    _, _, g1 = oracle.grid_d(ref, threads=8)
+    t = {k: torch.as_tensor(np.asarray(w[k], np.float32)).cuda()
+         for k in ("uu", "vv", "ww", "vis")}
+    lib = fg.load()
+    for radius in (0, 40):
+        ws = fg.Workspace(0)
+        cube = fg.Cube(ws, w["support"], 4, w["conv_size_half"],
+                       np.asarray(w["conv_func"], np.float32), False)
+        out = []
+        for accum, fail in ((_lib.ACCUM_PLAIN, -1),
+                            (_lib.ACCUM_COMPENSATED, 0),
+                            (_lib.ACCUM_COMPENSATED, -1)):
+            grid = torch.zeros(2 * w["grid_size"] ** 2, device="cuda")
+            torch.cuda.synchronize()
+            # (the plain job has sized everything but the sums)
+            assert lib.oskar_b200_testing_fail_allocation(fail) == _lib.OK
+            try:
+                fg.grid_device(ws, cube, t["uu"], t["vv"], t["ww"], t["vis"],
+                               None, 1.0, 1.0, w["grid_size"], grid,
+                               opts=fg.options(accum_mode=accum,
+                                               compensate_radius=radius))
+                torch.cuda.synchronize()
+            finally:
+                lib.oskar_b200_testing_fail_allocation(-1)
+            assert ws.stats().status == 0
+            out.append(grid.cpu().numpy())
+            assert oracle.rel_rms(out[-1], g1) <= 1e-5
+        # FP64 sums of FP32-rounded products, rounded to FP32 once: the two
+        # ways differ by the FP64 summation order before that rounding.
+        if radius == 0:
+            assert oracle.rel_rms(out[1], out[2]) <= 2e-7
+        cube.close()
+        ws.close()
