@@ -577,8 +577,8 @@ size_t oskar_b200_workspace_bytes(const oskar_B200Workspace* ws)
     if (!ws) return 0;
     const DeviceBuffer* bufs[] = {
         &ws->keys[0], &ws->keys[1], &ws->vals[0], &ws->vals[1], &ws->rec,
-        &ws->scan_tmp, &ws->flags, &ws->task_start, &ws->task_job,
-        &ws->counters, &ws->partials, &ws->plane_counts, &ws->in_uu,
+        &ws->sort_tmp, &ws->task_start, &ws->task_job,
+        &ws->counters, &ws->partials, &ws->in_uu,
         &ws->in_vv, &ws->in_ww, &ws->in_vis, &ws->in_weight, &ws->in_grid,
         &ws->in_cube, &ws->in_norm, &ws->comp_grid};
     size_t t = 0;
@@ -1127,6 +1127,9 @@ int weights_write_drop_in(size_t n, const T* uu, const T* vv,
     B200_PCHECK(cudaMemcpyAsync(skips.data(), d_skip,
                                 sizeof(unsigned long long) * chunks,
                                 cudaMemcpyDeviceToHost, s));
+    B200_PCHECK(cudaStreamSynchronize(s));
+    for (unsigned long long x : skips)
+        if (x == kSortFailed) return OSKAR_B200_ERR_TIMEOUT;
     B200_PCHECK(cudaMemcpyAsync(grid, ws->in_grid.ptr, grid_bytes,
                                 cudaMemcpyDeviceToHost, s));
     B200_PCHECK(cudaStreamSynchronize(s));

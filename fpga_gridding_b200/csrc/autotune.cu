@@ -218,7 +218,7 @@ int run_autotune(oskar_B200Workspace* ws, const oskar_B200Cube* cube,
     // above in use; the pipeline from prep to the end of gridding is timed.
     const bool comp = opt_in->accum_mode == OSKAR_B200_ACCUM_COMPENSATED;
     KeyLayout kl;
-    if (!make_key_layout(grid_size, P, 1, &kl))
+    if (!make_key_layout(grid_size, P, 1, n, &kl))
     {
         ws->stage_timing = saved_timing;
         return OSKAR_B200_ERR_UNSUPPORTED;

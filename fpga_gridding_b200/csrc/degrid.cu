@@ -20,6 +20,7 @@
 // original indices).
 #include "common.cuh"
 #include "internal.h"
+#include "prep.cuh"
 
 namespace b200 {
 namespace {
@@ -147,13 +148,15 @@ template <typename GT, typename KT>
 __global__ void __launch_bounds__(kDegridWarps * 32, 4)
 degrid_kernel(const uint32_t* __restrict__ order,
               const uint32_t* __restrict__ sorted_keys,
-              const int4* __restrict__ rec, const JobDesc* __restrict__ jobs,
+              const uint2* __restrict__ rec, const JobDesc* __restrict__ jobs,
               int job_shift, int apply_weight,
               unsigned long long* __restrict__ counters, size_t n)
 {
     using C2 = typename Cplx<GT>::type;
     __shared__ unsigned long long s_chunk;
-    const size_t valid = n - counters[CNT_SKIPPED];
+    // A sort that gave up leaves nothing to do.
+    const size_t valid = counters[CNT_STATUS] & DEV_ERR_TIMEOUT
+                             ? 0 : n - counters[CNT_SKIPPED];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int group = lane / kGroup, gl = lane % kGroup;
     // A CTA takes chunks of kDegridChunk consecutive sorted visibilities
@@ -183,7 +186,7 @@ degrid_kernel(const uint32_t* __restrict__ order,
             {
                 i = order[s];
                 jd = &jobs[sorted_keys[s] >> job_shift];
-                r = rec[i];
+                r = unpack_record(rec[i]);
             }
             int S = 0, W = 0, u0 = 0, v0 = 0, off_u = 0, off_v = 0, half = 0;
             int os = 1, G = 1;
@@ -299,7 +302,7 @@ degrid_kernel(const uint32_t* __restrict__ order,
 }  // namespace
 
 cudaError_t launch_degrid(const uint32_t* order, const uint32_t* sorted_keys,
-                          const int4* rec, const JobDesc* jobs, int job_shift,
+                          const uint2* rec, const JobDesc* jobs, int job_shift,
                           int apply_weight, unsigned long long* counters,
                           size_t n,
                           int data_is_double, int kernel_type, int num_sms,

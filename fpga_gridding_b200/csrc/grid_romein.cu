@@ -29,6 +29,7 @@
 #include "common.cuh"
 #include "grid_romein.cuh"
 #include "internal.h"
+#include "prep.cuh"
 
 namespace b200 {
 namespace {
@@ -659,7 +660,7 @@ romein_grid_kernel(const GridArgs a)
         {
             const uint32_t i = a.order[begin + t];
             RawVis<GT> rv;
-            rv.rec = a.rec[i];
+            rv.rec = unpack_record(a.rec[i]);
             const size_t local = i - jd.first;
             const GT* __restrict__ vis = static_cast<const GT*>(jd.vis);
             GT re = vis[2 * local], im = vis[2 * local + 1];

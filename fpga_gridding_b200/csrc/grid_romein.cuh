@@ -19,7 +19,7 @@ constexpr int kMaxOffsets = 33;     // 2 * ceil(oversample / 2) + 1, oversample 
 struct GridArgs
 {
     const uint32_t* order;      // sorted position -> point (global index)
-    const int4* rec;            // placement record of each point
+    const uint2* rec;           // placement record of each point
     int apply_weight;           // visibilities x weight (see JobDesc)
     const uint32_t* task_start; // [num_tasks + 1]
     const uint32_t* task_job;   // [num_tasks]: job of each task

@@ -126,11 +126,11 @@ struct oskar_B200Workspace
     size_t smem_optin = 0;
     cudaStream_t stream = nullptr;
     // per-visibility work arrays
-    b200::DeviceBuffer keys[2], vals[2], rec, scan_tmp, flags;
+    b200::DeviceBuffer keys[2], vals[2], rec, sort_tmp;
     b200::DeviceBuffer task_start, task_job;
-    // small arrays: counters, partial sums, per-job plane histograms and
-    // skip counts, the job table
-    b200::DeviceBuffer counters, partials, plane_counts, job_skipped, jobs;
+    // small arrays: what a call starts from zero (the counters first, then
+    // see run_batch), partial sums, the job table
+    b200::DeviceBuffer counters, partials, jobs;
     // pinned host copies of the job table (the sources of its uploads), a
     // ring of them so that a call rarely waits for an earlier call's upload,
     // each with the event after which that upload has read it
@@ -207,20 +207,21 @@ enum CounterSlot
     CNT_FLUSHES = 3,
     CNT_STATUS = 4,      // DEV_ERR_* bits
     CNT_UPDATES = 5,     // grid updates (taps) of gridded points
+    CNT_TASK_TILE = 6,   // ticket of the task list's tiles
     CNT_COUNT = 8
 };
 
 // ---- radix_sort.cu --------------------------------------------------------
-size_t scan_temp_bytes(size_t n);
-// Exclusive prefix sum of n uint32 values (out must not alias in).
-cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n,
-                               void* temp, cudaStream_t st, int* launches);
 size_t radix_sort_temp_bytes(size_t n);
-// Stable LSD sort of (key, value) pairs on the low num_bits of the keys.
-// The sorted pairs end in keys[*which] / vals[*which].
+// Stable LSD sort of (key, position) pairs on the low num_bits of the keys in
+// keys[0]; the values are the positions 0 .. n - 1.  The sorted pairs end in
+// keys[*which] / vals[*which].  *status: the device status word; when it has
+// DEV_ERR_TIMEOUT (set here when a bounded wait expires) the pairs are not to
+// be used.
 cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
-                             int num_bits, void* temp, cudaStream_t st,
-                             int* which, int* launches);
+                             int num_bits, void* temp,
+                             unsigned long long* status, int num_sms,
+                             cudaStream_t st, int* which, int* launches);
 
 // ---- cube.cu ----------------------------------------------------------------
 // d_conv_im == nullptr: d_conv_func is the interleaved complex cube;
@@ -256,7 +257,8 @@ struct KeyLayout
 // 64, at most the grid); 0 picks grid_size / 16.  num_groups: most distinct
 // supports of any job's cube; 0 groups by w-plane.
 bool make_key_layout(int grid_size, int num_planes, int num_jobs,
-                     KeyLayout* out, int tile_shift = 0, int num_groups = 0);
+                     size_t num_points, KeyLayout* out, int tile_shift = 0,
+                     int num_groups = 0);
 // Sets each plane's group and returns the groups' supports (ascending, at
 // most 128: supports are <= 127).
 std::vector<int> assign_groups(PlaneDesc* planes, int num_planes);
@@ -306,7 +308,7 @@ cudaError_t launch_slice_bounds(const unsigned long long* counters,
 
 // ---- degrid.cu ------------------------------------------------------------
 cudaError_t launch_degrid(const uint32_t* order, const uint32_t* sorted_keys,
-                          const int4* rec, const JobDesc* jobs, int job_shift,
+                          const uint2* rec, const JobDesc* jobs, int job_shift,
                           int apply_weight, unsigned long long* counters,
                           size_t n, int data_is_double, int kernel_type,
                           int num_sms, cudaStream_t st);
@@ -330,6 +332,9 @@ int measure_atomic_rate(oskar_B200Workspace* ws, void* grid, int grid_size,
                         int iters, double* updates_per_s);
 
 // ---- weights.cu -------------------------------------------------------------
+// Skip count left by an ordered write whose sort gave up (the grid is then
+// unchanged).
+constexpr unsigned long long kSortFailed = ~0ull;
 // Uniform weighting (utils/oskar_grid_weights.c:38-172) on device arrays.
 // *d_num_skipped (or a workspace counter when null) is reset, then counts.
 int run_weights_write(oskar_B200Workspace* ws, int data_is_double,

@@ -173,7 +173,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
                         (opt->staging == 1 ||
                          (opt->staging == 0 && !comp && ws->tuned_launch &&
                           ws->tuned_staging == 1));
-    if (!make_key_layout(max_grid, max_planes, num_jobs, &kl, tile_shift,
+    if (!make_key_layout(max_grid, max_planes, num_jobs, n, &kl, tile_shift,
                          staged ? 0 : max_groups))
         return OSKAR_B200_ERR_UNSUPPORTED;
     if (bands)
@@ -286,21 +286,25 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         comp_off += (size_t)h.grid_size * h.grid_size;
     }
     const int bpj = prep_blocks_per_job(max_points, num_jobs, ws->num_sms);
-    B200_TRY(ws->counters.ensure(sizeof(unsigned long long) * CNT_COUNT));
+    // What starts from zero, in one buffer and one memset: the counters, then
+    // per job the skip count, the plane histogram and the ticket of its prep
+    // blocks (a word each, of which half is used), then the task list's tile
+    // words.
+    const size_t zero_words = CNT_COUNT +
+                              (size_t)num_jobs * (2 + (size_t)max_planes) +
+                              task_tiles(n);
+    B200_TRY(ws->counters.ensure(sizeof(unsigned long long) * zero_words));
     B200_TRY(ws->jobs.ensure(job_bytes));
-    B200_TRY(ws->job_skipped.ensure(sizeof(unsigned long long) * num_jobs));
-    B200_TRY(ws->plane_counts.ensure(sizeof(unsigned long long) * num_jobs *
-                                     max_planes));
     B200_TRY(ws->partials.ensure(sizeof(double) * num_jobs * bpj));
     unsigned long long* counters =
         static_cast<unsigned long long*>(ws->counters.ptr);
+    unsigned long long* job_skipped = counters + CNT_COUNT;
+    unsigned long long* plane_counts = job_skipped + num_jobs;
+    unsigned long long* job_tickets =
+        plane_counts + (size_t)num_jobs * max_planes;
+    unsigned long long* task_state = job_tickets + num_jobs;
     B200_TRY(cudaMemsetAsync(counters, 0,
-                             sizeof(unsigned long long) * CNT_COUNT, st));
-    B200_TRY(cudaMemsetAsync(ws->job_skipped.ptr, 0,
-                             sizeof(unsigned long long) * num_jobs, st));
-    B200_TRY(cudaMemsetAsync(ws->plane_counts.ptr, 0,
-                             sizeof(unsigned long long) * num_jobs * max_planes,
-                             st));
+                             sizeof(unsigned long long) * zero_words, st));
     B200_TRY(cudaMemcpyAsync(ws->jobs.ptr, hj, job_bytes,
                              cudaMemcpyHostToDevice, st));
     {
@@ -322,15 +326,13 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         B200_TRY(ws->keys[1].ensure(4 * n));
         B200_TRY(ws->vals[0].ensure(4 * n));
         B200_TRY(ws->vals[1].ensure(4 * n));
-        B200_TRY(ws->rec.ensure(16 * n));
+        B200_TRY(ws->rec.ensure(sizeof(uint2) * n));
         if (!degrid)
         {
-            B200_TRY(ws->flags.ensure(8 * task_tiles(n)));
             B200_TRY(ws->task_start.ensure(4 * (n + 2)));
             B200_TRY(ws->task_job.ensure(4 * (n + 2)));
         }
-        B200_TRY(ws->scan_tmp.ensure(std::max(radix_sort_temp_bytes(n),
-                                              scan_temp_bytes(n))));
+        B200_TRY(ws->sort_tmp.ensure(radix_sort_temp_bytes(n)));
     }
 
     PrepArgs pa{};
@@ -341,31 +343,21 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     // (the norm is not a degridding output)
     pa.apply_weight = degrid ? 0 : opt->apply_weight;
     pa.key = kl;
-    pa.rec = static_cast<int4*>(ws->rec.ptr);
+    pa.rec = static_cast<uint2*>(ws->rec.ptr);
     uint32_t* keys[2] = {static_cast<uint32_t*>(ws->keys[0].ptr),
                          static_cast<uint32_t*>(ws->keys[1].ptr)};
     uint32_t* vals[2] = {static_cast<uint32_t*>(ws->vals[0].ptr),
                          static_cast<uint32_t*>(ws->vals[1].ptr)};
     pa.keys = keys[0];
-    pa.vals = vals[0];
     pa.counters = counters;
-    pa.job_skipped = static_cast<unsigned long long*>(ws->job_skipped.ptr);
+    pa.job_skipped = job_skipped;
     pa.norm_partials = static_cast<double*>(ws->partials.ptr);
-    pa.plane_counts = static_cast<unsigned long long*>(ws->plane_counts.ptr);
+    pa.plane_counts = plane_counts;
+    pa.job_tickets = reinterpret_cast<uint32_t*>(job_tickets);
 
     B200_TRY(mark(0));
-    if (n > 0)
-    {
-        B200_TRY(launch_prep(pa, dbl, opt->coord_mode, st));
-        launches += 1;
-    }
-    else
-    {
-        B200_TRY(cudaMemsetAsync(pa.norm_partials, 0,
-                                 sizeof(double) * num_jobs * bpj, st));
-    }
-    // Norms, skip counts and grid updates of every job (also when empty).
-    B200_TRY(launch_finalize_prep(pa, st));
+    // (Also without points: it publishes every job's norm and skip count.)
+    B200_TRY(launch_prep(pa, dbl, opt->coord_mode, st));
     launches += 1;
     B200_TRY(mark(1));
     if (n == 0)
@@ -384,7 +376,8 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
 
     int which = 0;
     B200_TRY(radix_sort_pairs(keys, vals, n, kl.total_bits + 1,
-                              ws->scan_tmp.ptr, st, &which, &launches));
+                              ws->sort_tmp.ptr, counters + CNT_STATUS,
+                              ws->num_sms, st, &which, &launches));
     B200_TRY(mark(2));
     if (degrid)
     {
@@ -405,8 +398,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         kl, num_jobs, jobs, bands ? n / bands->num_bands : n);
     B200_TRY(launch_tasks(keys[which], n, counters, 2 * kl.fine_bits,
                           kl.job_shift, sizes,
-                          static_cast<uint32_t*>(ws->flags.ptr),
-                          ws->scan_tmp.ptr,
+                          task_state,
                           static_cast<uint32_t*>(ws->task_start.ptr),
                           static_cast<uint32_t*>(ws->task_job.ptr), st,
                           &launches));

@@ -12,10 +12,20 @@
 
 namespace b200 {
 
-// Sort key bits (skip flag included) that the fine cell index may fill.
-// Coarser fine cells sort faster but grid slower: at plain_large, 24 bits
-// (three 8-bit passes) gave sort 2.17 -> 1.47 ms, gridding 20.3 -> 22.2 ms.
-constexpr int kKeyBits = 32;
+// Sort key bits (skip flag included) that the fine cell index may fill: whole
+// passes of the sort, enough to tell about four times as many places apart as
+// there are points.  More bits cost a pass; fewer put points of a wider block
+// into a task in arrival order, which its own sort cannot undo.  One B200, 32
+// -> 24 bits: 2.2 M points, sort 136 -> 108 us, gridding 516 -> 533; 3.4 M
+// 161 -> 124, 5070 -> 5074; 39.2 M 1361 -> 1039, 16199 -> 18779.  24 -> 16:
+// 10 thousand points, sort 38 -> 30 us, gridding 16.4 both; 0.24 M 46 -> 32,
+// 45 -> 68.
+static int key_bits(size_t num_points)
+{
+    int b = 2;
+    while ((size_t(1) << (b - 2)) < num_points && b < 32) ++b;
+    return std::min(32, (b + 7) / 8 * 8);
+}
 
 std::vector<int> assign_groups(PlaneDesc* planes, int num_planes)
 {
@@ -31,7 +41,8 @@ std::vector<int> assign_groups(PlaneDesc* planes, int num_planes)
 }
 
 bool make_key_layout(int grid_size, int num_planes, int num_jobs,
-                     KeyLayout* out, int tile_shift, int num_groups)
+                     size_t num_points, KeyLayout* out, int tile_shift,
+                     int num_groups)
 {
     KeyLayout k{};
     int gbits = 0;
@@ -55,7 +66,8 @@ bool make_key_layout(int grid_size, int num_planes, int num_jobs,
     // (The same jobs are refused whatever the grouping.)
     if (k.job_bits + 2 * k.coarse_bits + plane_bits + 1 > 32) return false;
     const int fixed = k.job_bits + 2 * k.coarse_bits + k.group_bits + 1;
-    while (fixed + 2 * k.fine_bits > kKeyBits && k.fine_bits > 0)
+    const int bits = key_bits(num_points);
+    while (fixed + 2 * k.fine_bits > bits && k.fine_bits > 0)
     {
         ++k.fine_shift;
         --k.fine_bits;
@@ -168,9 +180,7 @@ prep_kernel(const PrepArgs a)
         {
             if (keep)
             {
-                a.rec[g] = make_int4(p.gu, p.gv,
-                                     p.plane | (p.conj < 0 ? (int)0x80000000 : 0),
-                                     (p.off_u + half) | ((p.off_v + half) << 16));
+                a.rec[g] = pack_record(p, half);
                 a.keys[g] = make_key(a.key, job, p.gu, p.gv,
                                      a.key.by_plane
                                          ? p.plane : jd.planes[p.plane].group);
@@ -184,7 +194,6 @@ prep_kernel(const PrepArgs a)
             {
                 a.keys[g] = skip_key;
             }
-            a.vals[g] = (uint32_t)g;
         }
         skipped += in_range && !keep;
         // plane histogram, aggregated across equal planes in the warp
@@ -224,140 +233,189 @@ prep_kernel(const PrepArgs a)
         for (int p = threadIdx.x; p < num_planes; p += blockDim.x)
             if (s_hist[p])
                 atomicAdd(&job_hist[p], (unsigned long long)s_hist[p]);
-}
-
-// One block per job: sums the job's norm partials in a fixed order
-// (deterministic), adds them to the caller's norm, publishes the skip count,
-// and counts grid updates from the plane histogram.
-__global__ void finalize_prep_kernel(const PrepArgs a)
-{
-    const int job = blockIdx.x;
-    const JobDesc& jd = a.jobs[job];
-    __shared__ double s_v[32];
-    __shared__ unsigned long long s_u[32];
-    double t = 0.0;
-    for (int i = threadIdx.x; i < a.blocks_per_job; i += blockDim.x)
-        t += a.norm_partials[(size_t)job * a.blocks_per_job + i];
-    unsigned long long up = 0;
-    const unsigned long long* hist = a.plane_counts + (size_t)job * a.max_planes;
-    for (int p = threadIdx.x; p < jd.num_planes; p += blockDim.x)
+    // The job's last block sums its norm partials in a fixed order
+    // (deterministic), adds them to the caller's norm, publishes the skip
+    // count, and counts grid updates from the plane histogram.  (As a kernel
+    // of its own this took a launch and 4 us.)
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        s_last = atomicAdd(&a.job_tickets[job], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    __shared__ unsigned long long s_updates[kPrepThreads / 32];
+    norm = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += kPrepThreads)
+        norm += __ldcg(&a.norm_partials[(size_t)job * gridDim.x + k]);
+    unsigned long long updates = 0;
+    for (int p = threadIdx.x; p < num_planes; p += kPrepThreads)
     {
         const unsigned long long w = 2ull * jd.support[p] + 1ull;
-        up += hist[p] * w * w;
+        updates += __ldcg(&job_hist[p]) * w * w;
     }
-    t = warp_sum(t);
-    up = warp_sum(up);
-    if ((threadIdx.x & 31) == 0)
+    norm = warp_sum(norm);
+    updates = warp_sum(updates);
+    if (lane == 0)
     {
-        s_v[threadIdx.x >> 5] = t;
-        s_u[threadIdx.x >> 5] = up;
+        s_norm[threadIdx.x >> 5] = norm;
+        s_updates[threadIdx.x >> 5] = updates;
     }
     __syncthreads();
     if (threadIdx.x == 0)
     {
-        double s = 0.0;
+        double t = 0.0;
         unsigned long long u = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
+        for (int w = 0; w < kPrepThreads / 32; ++w)
         {
-            s += s_v[w];
-            u += s_u[w];
+            t += s_norm[w];
+            u += s_updates[w];
         }
-        if (jd.d_norm) *jd.d_norm += s;
-        if (jd.d_skipped) *jd.d_skipped = a.job_skipped[job];
+        if (jd.d_norm) *jd.d_norm += t;
+        if (jd.d_skipped) *jd.d_skipped = __ldcg(&a.job_skipped[job]);
         atomicAdd(&a.counters[CNT_UPDATES], u);
     }
 }
 
-// Task list in two passes over the sorted keys, tiles of kTaskTile
-// positions: each tile counts its task starts, the tile counts are scanned,
-// and each tile writes its starts at its offset.  A task starts at sorted
-// position s < valid when s == 0, at every multiple of its group's task size,
-// or where the key above the fine cell bits changes.
+// Task list in one pass over the sorted keys, in tiles of kTaskTile positions:
+// each tile counts its task starts, finds the starts of the tiles before it by
+// chained scan (a tile's word holds its own count until it knows the sum up to
+// it; 32 earlier words are read at once) and writes its starts.  A task starts
+// at sorted position s < valid when s == 0, at every multiple of its group's
+// task size, or where the key above the fine cell bits changes.  (Counting,
+// a three-launch scan and writing took 34 us for 10 thousand points and 260 us
+// for 39 M.)
 constexpr int kTaskTile = 4096;
 constexpr int kTaskThreads = 256;
+constexpr int kTaskRounds = kTaskTile / kTaskThreads;
+constexpr int kTaskWarps = kTaskThreads / 32;
 
-__device__ __forceinline__ bool task_starts_at(const uint32_t* keys, size_t s,
-                                               size_t valid, int fine_bits,
-                                               const TaskSizes& sizes)
+// Sum of tile words [0, tile) by one warp; false when the bounded wait
+// expired.  Word: flag (1: the tile's count, 2: all tiles up to it) << 62 |
+// count.
+__device__ __forceinline__ bool tasks_before(const unsigned long long* state,
+                                             unsigned tile, unsigned* sum)
 {
-    return s < valid &&
-           (s == 0 ||
-            (s & ((1u << sizes.log2_max[(keys[s] >> fine_bits) &
-                                        sizes.group_mask]) - 1u)) == 0 ||
-            (keys[s] >> fine_bits) != (keys[s - 1] >> fine_bits));
+    const int lane = threadIdx.x & 31;
+    unsigned total = 0, end = tile, spins = 0;
+    while (end > 0)
+    {
+        const unsigned long long w =
+            (unsigned)lane < end
+                ? *((const volatile unsigned long long*)state + (end - 1 - lane))
+                : 2ull << 62;
+        const unsigned pending = __ballot_sync(0xffffffffu, (w >> 62) == 0);
+        const unsigned prefix = __ballot_sync(0xffffffffu, (w >> 62) == 2);
+        // words before the first pending one, up to the first prefix
+        const int usable = min(pending ? __ffs(pending) - 1 : 32,
+                               prefix ? __ffs(prefix) : 32);
+        total += __reduce_add_sync(
+            0xffffffffu, lane < usable ? (unsigned)(w & 0xffffffffull) : 0u);
+        if (prefix && __ffs(prefix) <= usable) break;
+        end -= (unsigned)usable;
+        if (usable == 0 && ++spins > kSpinLimit) return false;
+    }
+    *sum = total;
+    return true;
 }
 
 __global__ void __launch_bounds__(kTaskThreads)
-task_count_kernel(const uint32_t* __restrict__ keys, size_t n,
-                  const unsigned long long* __restrict__ counters,
-                  int fine_key_bits, const TaskSizes sizes,
-                  uint32_t* __restrict__ tile_counts)
+task_list_kernel(const uint32_t* __restrict__ keys, size_t n,
+                 unsigned long long* __restrict__ counters, int fine_key_bits,
+                 const TaskSizes sizes, int job_shift,
+                 unsigned long long* state, uint32_t* __restrict__ task_start,
+                 uint32_t* __restrict__ task_job)
 {
-    const size_t valid = n - counters[CNT_SKIPPED];
-    const size_t tile0 = (size_t)blockIdx.x * kTaskTile;
-    unsigned c = 0;
-    for (int k = threadIdx.x; k < kTaskTile; k += kTaskThreads)
-        c += task_starts_at(keys, tile0 + k, valid, fine_key_bits, sizes);
-    c = warp_sum(c);
-    __shared__ unsigned s_w[kTaskThreads / 32];
-    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = c;
-    __syncthreads();
+    __shared__ unsigned s_tile, s_base;
+    __shared__ unsigned s_w[kTaskRounds][kTaskWarps];
+    // A sort that gave up leaves no tasks (counters[CNT_TASKS] stays zero).
     if (threadIdx.x == 0)
-    {
-        unsigned t = 0;
-        for (int w = 0; w < kTaskThreads / 32; ++w) t += s_w[w];
-        tile_counts[blockIdx.x] = t;
-    }
-}
-
-// tile_offsets: exclusive scan of tile_counts (the last tile also needs its
-// own count to close the list).
-__global__ void __launch_bounds__(kTaskThreads)
-task_write_kernel(const uint32_t* __restrict__ keys, size_t n,
-                  unsigned long long* __restrict__ counters,
-                  int fine_key_bits, const TaskSizes sizes, int job_shift,
-                  const uint32_t* __restrict__ tile_counts,
-                  const uint32_t* __restrict__ tile_offsets,
-                  uint32_t* __restrict__ task_start,
-                  uint32_t* __restrict__ task_job)
-{
+        s_tile = counters[CNT_STATUS] & DEV_ERR_TIMEOUT
+                     ? 0xffffffffu
+                     : (unsigned)atomicAdd(&counters[CNT_TASK_TILE], 1ull);
+    __syncthreads();
+    const unsigned tile = s_tile;
+    if (tile == 0xffffffffu) return;
     const size_t valid = n - counters[CNT_SKIPPED];
-    const size_t tile0 = (size_t)blockIdx.x * kTaskTile;
+    const size_t tile0 = (size_t)tile * kTaskTile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __shared__ unsigned s_w[kTaskThreads / 32];
-    uint32_t base = tile_offsets[blockIdx.x];
     // rounds of kTaskThreads consecutive positions, in order
-    for (int r = 0; r < kTaskTile; r += kTaskThreads)
-    {
-        const size_t pos = tile0 + r + threadIdx.x;
-        const bool f = task_starts_at(keys, pos, valid, fine_key_bits, sizes);
-        const unsigned ball = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) s_w[warp] = __popc(ball);
-        __syncthreads();
-        unsigned before = 0, total = 0;
+    unsigned ball[kTaskRounds];
+    uint32_t key[kTaskRounds], edge[kTaskRounds];
 #pragma unroll
-        for (int w = 0; w < kTaskThreads / 32; ++w)
-        {
-            before += w < warp ? s_w[w] : 0u;
-            total += s_w[w];
-        }
-        if (f)
-        {
-            const uint32_t t = base + before +
-                               __popc(ball & ((1u << lane) - 1u));
-            task_start[t] = (uint32_t)pos;
-            task_job[t] = keys[pos] >> job_shift;
-        }
-        base += total;
-        __syncthreads();   // s_w is rewritten by the next round
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+    for (int r = 0; r < kTaskRounds; ++r)
     {
-        const uint32_t num_tasks = tile_offsets[blockIdx.x] +
-                                   tile_counts[blockIdx.x];
-        counters[CNT_TASKS] = num_tasks;
-        task_start[num_tasks] = (uint32_t)valid;
+        const size_t s = tile0 + (size_t)r * kTaskThreads + threadIdx.x;
+        key[r] = s < valid ? keys[s] : 0u;
+        edge[r] = lane == 0 && s > 0 && s < valid ? keys[s - 1] : 0u;
     }
+#pragma unroll
+    for (int r = 0; r < kTaskRounds; ++r)
+    {
+        const size_t s = tile0 + (size_t)r * kTaskThreads + threadIdx.x;
+        const uint32_t up = __shfl_up_sync(0xffffffffu, key[r], 1);
+        const uint32_t prev = (lane ? up : edge[r]) >> fine_key_bits;
+        const uint32_t k = key[r] >> fine_key_bits;
+        const uint32_t low =
+            (1u << sizes.log2_max[k & sizes.group_mask]) - 1u;
+        ball[r] = __ballot_sync(0xffffffffu, s < valid &&
+                                (s == 0 || k != prev ||
+                                 ((uint32_t)s & low) == 0));
+        if (lane == 0) s_w[r][warp] = __popc(ball[r]);
+    }
+    __syncthreads();
+    if (warp == 0)
+    {
+        // Exclusive scan of the tile's warp counts, 4 per lane.
+        static_assert(kTaskRounds * kTaskWarps == 128, "4 counts per lane");
+        unsigned* w = &s_w[0][0] + 4 * lane;
+        const unsigned c0 = w[0], c1 = w[1], c2 = w[2], c3 = w[3];
+        unsigned inc = c0 + c1 + c2 + c3;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const unsigned t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        const unsigned ex = inc - (c0 + c1 + c2 + c3);
+        w[0] = ex;
+        w[1] = ex + c0;
+        w[2] = ex + c0 + c1;
+        w[3] = ex + c0 + c1 + c2;
+        const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
+        volatile unsigned long long* word = state + tile;
+        if (lane == 0) *word = (tile ? 1ull : 2ull) << 62 | total;
+        unsigned before = 0;
+        const bool ok = tasks_before(state, tile, &before);
+        if (lane == 0)
+        {
+            if (ok)
+                *word = 2ull << 62 | (before + total);
+            else
+                atomicOr(&counters[CNT_STATUS],
+                         (unsigned long long)DEV_ERR_TIMEOUT);
+            s_base = ok ? before : 0xffffffffu;
+            if (ok && tile == gridDim.x - 1)
+            {
+                counters[CNT_TASKS] = before + total;
+                task_start[before + total] = (uint32_t)valid;
+            }
+        }
+    }
+    __syncthreads();
+    const unsigned base = s_base;
+    if (base == 0xffffffffu) return;
+#pragma unroll
+    for (int r = 0; r < kTaskRounds; ++r)
+        if ((ball[r] >> lane) & 1u)
+        {
+            const size_t pos = tile0 + (size_t)r * kTaskThreads + threadIdx.x;
+            const uint32_t t = base + s_w[r][warp] +
+                               __popc(ball[r] & ((1u << lane) - 1u));
+            task_start[t] = (uint32_t)pos;
+            task_job[t] = key[r] >> job_shift;
+        }
 }
 
 // Placement only, for inspection (oskar_b200_place).
@@ -405,32 +463,20 @@ cudaError_t launch_prep(const PrepArgs& a, int data_is_double, int coord_mode,
     return cudaGetLastError();
 }
 
-cudaError_t launch_finalize_prep(const PrepArgs& a, cudaStream_t st)
-{
-    finalize_prep_kernel<<<a.num_jobs, 256, 0, st>>>(a);
-    return cudaGetLastError();
-}
-
 size_t task_tiles(size_t n) { return (n + kTaskTile - 1) / kTaskTile; }
 
 cudaError_t launch_tasks(const uint32_t* sorted_keys, size_t n,
                          unsigned long long* counters, int fine_key_bits,
                          int job_shift, const TaskSizes& sizes,
-                         uint32_t* tile_counts, void* scan_tmp, uint32_t* task_start,
+                         unsigned long long* tile_state, uint32_t* task_start,
                          uint32_t* task_job, cudaStream_t st, int* launches)
 {
     const size_t tiles = task_tiles(n);
     if (tiles == 0) return cudaSuccess;
-    uint32_t* tile_offsets = tile_counts + tiles;
-    task_count_kernel<<<(unsigned)tiles, kTaskThreads, 0, st>>>(
-        sorted_keys, n, counters, fine_key_bits, sizes, tile_counts);
-    cudaError_t e = exclusive_scan_u32(tile_counts, tile_offsets, tiles,
-                                       scan_tmp, st, launches);
-    if (e != cudaSuccess) return e;
-    if (launches) *launches += 2;
-    task_write_kernel<<<(unsigned)tiles, kTaskThreads, 0, st>>>(
-        sorted_keys, n, counters, fine_key_bits, sizes, job_shift,
-        tile_counts, tile_offsets, task_start, task_job);
+    if (launches) *launches += 1;
+    task_list_kernel<<<(unsigned)tiles, kTaskThreads, 0, st>>>(
+        sorted_keys, n, counters, fine_key_bits, sizes, job_shift, tile_state,
+        task_start, task_job);
     return cudaGetLastError();
 }
 

@@ -114,6 +114,27 @@ __device__ __forceinline__ float scale_coord(float x, const JobDesc& jd)
     return __fmul_rn(x, jd.coord_scale_f);
 }
 
+// Placement record of a kept point, 8 bytes: x = gu | gv << 16 (grids are at
+// most 65535 wide), y = plane | (w > 0) << 15 | (off_u + H) << 16 |
+// (off_v + H) << 22 (at most 2^15 planes, offsets + H at most 32).  Against
+// 16-byte records: 8 bytes less to write and to gather per point.
+__device__ __forceinline__ uint2 pack_record(const Placed& p, int half)
+{
+    return make_uint2((uint32_t)p.gu | ((uint32_t)p.gv << 16),
+                      (uint32_t)p.plane | (p.conj < 0 ? 1u << 15 : 0u) |
+                          ((uint32_t)(p.off_u + half) << 16) |
+                          ((uint32_t)(p.off_v + half) << 22));
+}
+
+// As the kernels use it: {gu, gv, plane | (w > 0) << 31,
+// (off_u + H) | (off_v + H) << 16}.
+__device__ __forceinline__ int4 unpack_record(const uint2 r)
+{
+    return make_int4((int)(r.x & 0xffffu), (int)(r.x >> 16),
+                     (int)((r.y & 0x7fffu) | ((r.y & 0x8000u) << 16)),
+                     (int)(((r.y >> 16) & 0x3fu) | ((r.y >> 22) << 16)));
+}
+
 // Prep of a batch: launch grid (blocks_per_job, num_jobs), block (x, j)
 // walks job j's points.
 struct PrepArgs
@@ -124,31 +145,30 @@ struct PrepArgs
     int max_planes;          // row stride of plane_counts
     int apply_weight;
     KeyLayout key;
-    int4* rec;               // [total points], global index
+    uint2* rec;              // [total points], global index
     uint32_t* keys;
-    uint32_t* vals;
     unsigned long long* counters;     // CNT_SKIPPED: all jobs
     unsigned long long* job_skipped;  // [num_jobs]
     double* norm_partials;            // [num_jobs][blocks_per_job]
     unsigned long long* plane_counts; // [num_jobs][max_planes]
+    uint32_t* job_tickets;            // [num_jobs]: blocks that are done
 };
 
 // Blocks per job: about 8 per SM over the whole batch, at least one per job,
 // no more than the largest job needs.
 int prep_blocks_per_job(size_t max_points, int num_jobs, int num_sms);
+// The last block of each job adds the job's partials to its norm and publishes
+// its skip count and grid updates.  (Also for jobs without points.)
 cudaError_t launch_prep(const PrepArgs& a, int data_is_double, int coord_mode,
                         cudaStream_t st);
-// Per job: norm += sum of its partials; skip count; grid updates.
-cudaError_t launch_finalize_prep(const PrepArgs& a, cudaStream_t st);
 // Task list: a task starts where (job, coarse tile, group) changes and every
-// 2^log2_max positions; task_job[t] is the job of task t.  tile_counts holds
-// 2 * task_tiles(n) entries; scan_tmp as exclusive_scan_u32 needs for
-// task_tiles(n) values.
+// 2^log2_max positions; task_job[t] is the job of task t.  tile_state: a zeroed
+// word per tile (task_tiles(n)); counters[CNT_TASK_TILE] is zero.
 size_t task_tiles(size_t n);
 cudaError_t launch_tasks(const uint32_t* sorted_keys, size_t n,
                          unsigned long long* counters, int fine_key_bits,
                          int job_shift, const TaskSizes& sizes,
-                         uint32_t* tile_counts, void* scan_tmp, uint32_t* task_start,
+                         unsigned long long* tile_state, uint32_t* task_start,
                          uint32_t* task_job, cudaStream_t st, int* launches);
 // Bands of a single job's task list: band b holds the tasks of coarse-tile
 // row b; band_first[b] (b <= num_bands) is its first task.

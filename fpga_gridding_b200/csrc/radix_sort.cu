@@ -1,44 +1,69 @@
-// Device prefix sum and stable LSD radix sort of (uint32 key, uint32 value)
-// pairs, written for this project (no CUB).
+// Stable LSD radix sort of (uint32 key, uint32 value) pairs, written for this
+// project (no CUB).
 //
-// Radix sort: 8-bit digits, one pass per digit.  Each pass is
-//   1. rs_histogram: per 4096-key tile, per-digit counts, stored digit-major
-//      (counts[digit * num_tiles + tile]);
-//   2. exclusive scan of that array: the output position of the first key of
-//      each (digit, tile);
-//   3. rs_scatter: stable ranks inside the tile, the tile's pairs reordered
-//      digit-major in shared memory, then written out as one contiguous run
-//      per digit (coalesced; scattering each pair straight to its bucket
-//      made every warp store touch 32 sectors: 2.70 -> 2.19 ms for the four
-//      passes over 39 M pairs).
-// Inside a tile each warp owns a contiguous run of 512 keys, read as 16
-// coalesced 32-key rows.  Equal digits in a row are ranked with
-// __match_any_sync against warp-private running counts, so the whole tile
-// needs only two block barriers.
+// One-sweep form: rs_histogram counts the digits of every pass in one read of
+// the keys; then each 8-bit digit takes one launch, in which a tile of 4096
+// pairs ranks its keys, publishes its digit counts, finds the counts of the
+// tiles before it by decoupled look-back (Merrill and Garland's chained scan:
+// a tile's word holds its own count until it knows the sum of all tiles up to
+// it) and writes its pairs.  What a pass must move is 16 bytes per pair; a
+// histogram, a three-launch scan and a scatter per digit (20 launches for 32
+// bits) took 2.16 ms for 39 M pairs and 80 us for 10 thousand.
+//
+// Inside a tile each of 16 warps owns a contiguous run of 256 keys, read as 8
+// coalesced rows of 32.  Lanes with equal digits find each other through a
+// mask word per digit in shared memory; the running counts are private to the
+// warp, so ranks need no block barrier.  The tile's pairs are put in digit
+// order in shared memory and leave as one contiguous run per digit.  A pass is
+// bound by the latency of that chain, so what counts is warps in flight: 39 M
+// pairs, 4 passes, 8 warps of 16 rows (126 registers) 2.21 ms, 16 warps of 8
+// rows at 3 blocks per SM 1.36 (1.46 at 2 blocks, 1.34 at 4 with spills);
+// __match_any_sync instead of the mask words 2.35 against 2.21 ms.
+//
+// A look-back waits only for tiles with smaller tickets, which are running
+// already.  The wait is bounded all the same: when it expires the sort sets
+// DEV_ERR_TIMEOUT in the status word and writes nothing more, and the kernels
+// that read the sorted pairs do nothing when that bit is set.
 #include "common.cuh"
 #include "internal.h"
 
 namespace b200 {
 namespace {
 
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;  // 2048
-
-constexpr int kSortThreads = 256;
+constexpr int kSortThreads = 512;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;
+constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;  // 4096
 constexpr int kRadix = 256;
+constexpr int kHistThreads = 256;
+constexpr int kMaxPasses = 4;
+constexpr int kLookback = 8;   // tiles read at once
 
-// ---------------------------------------------------------------------------
-// Scan
-// ---------------------------------------------------------------------------
+// Scratch: tile words of one pass (see look_back), then the digit counts of
+// every pass, turned into the digits' first positions by the histogram's last
+// block, then one ticket per pass and the histogram's.
+struct SortTemp
+{
+    unsigned long long* state;
+    uint32_t* digits;     // [kMaxPasses][kRadix]
+    uint32_t* tickets;    // [kMaxPasses + 1]
+};
 
-// Block-wide exclusive scan of one value per thread; returns the block total.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v,
-                                                         uint32_t* s_warp,
-                                                         uint32_t* total)
+size_t sort_tiles(size_t n) { return (n + kSortTile - 1) / kSortTile; }
+
+SortTemp sort_temp(void* temp, size_t n)
+{
+    SortTemp t;
+    t.state = static_cast<unsigned long long*>(temp);
+    t.digits = reinterpret_cast<uint32_t*>(t.state + sort_tiles(n) * kRadix);
+    t.tickets = t.digits + kMaxPasses * kRadix;
+    return t;
+}
+
+// Exclusive scan of one value per thread over the block's first kRadix
+// threads (all threads call it).
+__device__ __forceinline__ uint32_t digit_exclusive_scan(uint32_t v,
+                                                         uint32_t* s_warp)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t inc = v;
@@ -48,272 +73,299 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v,
         const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += t;
     }
-    if (lane == 31) s_warp[warp] = inc;
+    if (lane == 31 && warp < kRadix / 32) s_warp[warp] = inc;
     __syncthreads();
-    if (warp == 0)
-    {
-        uint32_t w = lane < (int)(blockDim.x >> 5) ? s_warp[lane] : 0;
-        uint32_t wi = w;
+    uint32_t before = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += t;
-        }
-        if (lane < (int)(blockDim.x >> 5)) s_warp[lane] = wi - w;
-        if (lane == 31) *total = wi;
-    }
+    for (int w = 0; w < kRadix / 32; ++w) before += w < warp ? s_warp[w] : 0u;
     __syncthreads();
-    return s_warp[warp] + inc - v;
+    return before + inc - v;
 }
 
-__global__ void __launch_bounds__(kScanThreads)
-scan_reduce_kernel(const uint32_t* __restrict__ in, size_t n,
-                   uint32_t* __restrict__ block_sums)
+// Digit counts of every pass; the last block turns them into the digits'
+// first positions.
+__global__ void __launch_bounds__(kHistThreads)
+rs_histogram_kernel(const uint32_t* __restrict__ keys, size_t n, int num_bits,
+                    SortTemp t)
 {
-    const size_t base = (size_t)blockIdx.x * kScanTile;
-    uint32_t s = 0;
+    __shared__ uint32_t s_count[kMaxPasses][kRadix];
+    __shared__ uint32_t s_warp[kRadix / 32];
+    __shared__ unsigned s_last;
+    const int passes = (num_bits + 7) / 8;
+    for (int i = threadIdx.x; i < kMaxPasses * kRadix; i += kHistThreads)
+        (&s_count[0][0])[i] = 0;
+    __syncthreads();
+    const uint32_t top = (1u << (num_bits - 8 * (passes - 1))) - 1u;
+    auto count = [&](uint32_t k) {
 #pragma unroll
-    for (int i = 0; i < kScanItems; ++i)
+        for (int p = 0; p < kMaxPasses; ++p)
+            if (p < passes)
+                atomicAdd(&s_count[p][(k >> (8 * p)) &
+                                      (p == passes - 1 ? top : 0xffu)], 1u);
+    };
+    // (the key buffers are at least 16-byte aligned)
+    const uint4* keys4 = reinterpret_cast<const uint4*>(keys);
+    const size_t stride = (size_t)gridDim.x * kHistThreads;
+    const size_t first = (size_t)blockIdx.x * kHistThreads + threadIdx.x;
+    size_t i = first;
+    for (; i + stride < n / 4; i += 2 * stride)
     {
-        const size_t p = base + (size_t)i * kScanThreads + threadIdx.x;
-        if (p < n) s += in[p];
+        const uint4 a = keys4[i], b = keys4[i + stride];
+        count(a.x); count(a.y); count(a.z); count(a.w);
+        count(b.x); count(b.y); count(b.z); count(b.w);
     }
-    s = warp_sum(s);
-    __shared__ uint32_t s_w[kScanThreads / 32];
-    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = s;
+    for (; i < n / 4; i += stride)
+    {
+        const uint4 a = keys4[i];
+        count(a.x); count(a.y); count(a.z); count(a.w);
+    }
+    if (first < n % 4) count(keys[n - 1 - first]);
+    __syncthreads();
+    static_assert(kRadix == kHistThreads, "one digit per thread");
+    for (int p = 0; p < passes; ++p)
+    {
+        const uint32_t c = s_count[p][threadIdx.x];
+        if (c) atomicAdd(&t.digits[p * kRadix + threadIdx.x], c);
+    }
+    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0)
+        s_last = atomicAdd(&t.tickets[kMaxPasses], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int p = 0; p < passes; ++p)
     {
-        uint32_t t = 0;
-        for (int w = 0; w < kScanThreads / 32; ++w) t += s_w[w];
-        block_sums[blockIdx.x] = t;
+        uint32_t* d = t.digits + p * kRadix + threadIdx.x;
+        *d = digit_exclusive_scan(__ldcg(d), s_warp);
     }
 }
 
-// One block scans the block sums in place (exclusive).
-__global__ void __launch_bounds__(1024)
-scan_block_sums_kernel(uint32_t* __restrict__ sums, size_t count)
+// Tile words: flag (2 bits) | pass + 1 (8 bits) | count.  The pass tells the
+// words of this pass from those left by the one before.
+constexpr unsigned long long kTileSum = 1ull << 62;        // this tile's count
+constexpr unsigned long long kTilePrefix = 2ull << 62;     // all tiles up to it
+constexpr unsigned long long kTileCount = (1ull << 40) - 1;
+
+__device__ __forceinline__ unsigned long long load_word(
+    const unsigned long long* p)
 {
-    __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_total;
-    uint32_t carry = 0;
-    for (size_t base = 0; base < count; base += blockDim.x)
-    {
-        const size_t p = base + threadIdx.x;
-        const uint32_t v = p < count ? sums[p] : 0;
-        const uint32_t ex = block_exclusive_scan(v, s_warp, &s_total);
-        if (p < count) sums[p] = carry + ex;
-        carry += s_total;
-        __syncthreads();
-    }
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p)
+                 : "memory");
+    return v;
 }
 
-__global__ void __launch_bounds__(kScanThreads)
-scan_apply_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
-                  size_t n, const uint32_t* __restrict__ block_offsets)
+__device__ __forceinline__ void store_word(unsigned long long* p,
+                                           unsigned long long v)
 {
-    __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_total;
-    // Thread t scans items [t * 8, t * 8 + 8) of the tile.
-    const size_t base = (size_t)blockIdx.x * kScanTile +
-                        (size_t)threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v)
+                 : "memory");
+}
+
+// Sum of the counts of tiles [0, tile), for the word column `col` (stride
+// words per tile); false when the bounded wait expired.
+__device__ __forceinline__ bool look_back(const unsigned long long* col,
+                                          size_t stride, size_t tile,
+                                          unsigned tag, uint32_t* sum)
+{
     uint32_t s = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; ++i)
+    size_t end = tile;   // tiles [0, end) are still to be added
+    unsigned spins = 0;
+    bool done = tile == 0;
+    while (!done)
     {
-        v[i] = (base + i < n) ? in[base + i] : 0;
-        s += v[i];
-    }
-    uint32_t run = block_exclusive_scan(s, s_warp, &s_total) +
-                   block_offsets[blockIdx.x];
+        unsigned long long w[kLookback];
 #pragma unroll
-    for (int i = 0; i < kScanItems; ++i)
-    {
-        if (base + i < n) out[base + i] = run;
-        run += v[i];
+        for (int j = 0; j < kLookback; ++j)
+            w[j] = end > (size_t)j ? load_word(col + (end - 1 - j) * stride)
+                                   : 0ull;
+        int used = 0;
+        bool ready = true;
+#pragma unroll
+        for (int j = 0; j < kLookback; ++j)
+        {
+            ready = ready && !done && (w[j] >> 62) != 0 &&
+                    ((w[j] >> 40) & 0xffu) == tag;
+            if (ready)
+            {
+                s += (uint32_t)(w[j] & kTileCount);
+                ++used;
+                done = (w[j] >> 62) == 2;
+            }
+        }
+        end -= used;
+        if (used == 0 && ++spins > kSpinLimit) return false;
     }
+    *sum = s;
+    return true;
 }
 
-// ---------------------------------------------------------------------------
-// Radix sort passes
-// ---------------------------------------------------------------------------
-
-__global__ void __launch_bounds__(kSortThreads)
-rs_histogram_kernel(const uint32_t* __restrict__ keys, size_t n, int shift,
-                    uint32_t mask, size_t num_tiles,
-                    uint32_t* __restrict__ counts)
+// One pass.  vals_in null: the values are the positions 0 .. n - 1.
+__global__ void __launch_bounds__(kSortThreads, 3)
+rs_pass_kernel(const uint32_t* __restrict__ keys_in,
+               const uint32_t* __restrict__ vals_in, size_t n, int pass,
+               uint32_t mask, SortTemp t, unsigned long long* status,
+               uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out)
 {
-    __shared__ uint32_t s_count[kSortWarps][kRadix];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads)
-        (&s_count[0][0])[i] = 0;
-    __syncthreads();
-    const size_t base = (size_t)blockIdx.x * kSortTile +
-                        (size_t)warp * (32 * kSortItems);
-#pragma unroll 4
-    for (int i = 0; i < kSortItems; ++i)
-    {
-        const size_t p = base + (size_t)i * 32 + lane;
-        const unsigned d = p < n ? ((keys[p] >> shift) & mask) : kRadix;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        if (d < kRadix && lane == __ffs(peers) - 1)
-            s_count[warp][d] += __popc(peers);
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < kRadix; d += kSortThreads)
-    {
-        uint32_t t = 0;
-#pragma unroll
-        for (int w = 0; w < kSortWarps; ++w) t += s_count[w][d];
-        counts[(size_t)d * num_tiles + blockIdx.x] = t;
-    }
-}
-
-__global__ void __launch_bounds__(kSortThreads)
-rs_scatter_kernel(const uint32_t* __restrict__ keys_in,
-                  const uint32_t* __restrict__ vals_in, size_t n, int shift,
-                  uint32_t mask, size_t num_tiles,
-                  const uint32_t* __restrict__ offsets,
-                  uint32_t* __restrict__ keys_out,
-                  uint32_t* __restrict__ vals_out)
-{
-    __shared__ uint32_t s_count[kSortWarps][kRadix];
-    // the tile's pairs in digit-major (stable) order, then written out in
-    // contiguous runs per digit
+    __shared__ uint16_t s_count[kSortWarps][kRadix];
+    // The tile's pairs in digit order; before that, the lanes of each warp
+    // that hold a digit.
     __shared__ uint32_t s_keys[kSortTile], s_vals[kSortTile];
-    __shared__ uint32_t s_digit_start[kRadix];   // within the tile
-    __shared__ uint32_t s_digit_out[kRadix];     // global position
-    __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_total;
+    uint32_t (*s_peers)[kRadix] = reinterpret_cast<uint32_t (*)[kRadix]>(s_keys);
+    static_assert(kSortWarps * kRadix <= kSortTile, "peer masks fit");
+    __shared__ uint32_t s_out[kRadix];   // global minus in-tile position
+    __shared__ uint32_t s_warp[kRadix / 32];
+    __shared__ unsigned s_tile;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const int shift = 8 * pass;
+    if (threadIdx.x == 0)
+        s_tile = (load_word(status) & DEV_ERR_TIMEOUT)
+                     ? 0xffffffffu : atomicAdd(&t.tickets[pass], 1u);
     for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads)
+    {
         (&s_count[0][0])[i] = 0;
+        (&s_peers[0][0])[i] = 0;
+    }
     __syncthreads();
-
-    const size_t tile0 = (size_t)blockIdx.x * kSortTile;
-    const size_t base = tile0 + (size_t)warp * (32 * kSortItems);
-    uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+    if (s_tile == 0xffffffffu) return;   // an earlier pass gave up
+    const size_t tile = s_tile, tile0 = tile * kSortTile;
+    const int tile_n = (int)min((size_t)kSortTile, n - tile0);
+    const int base = warp * (32 * kSortItems) + lane;
+    uint32_t key[kSortItems], rank[kSortItems];
+    keys_in += tile0 + base;
+#pragma unroll
+    for (int i = 0; i < kSortItems; ++i)
+        key[i] = base + i * 32 < tile_n ? keys_in[i * 32] : 0u;
 #pragma unroll
     for (int i = 0; i < kSortItems; ++i)
     {
-        const size_t p = base + (size_t)i * 32 + lane;
-        const bool ok = p < n;
-        key[i] = ok ? keys_in[p] : 0u;
-        val[i] = ok ? vals_in[p] : 0u;
-        const unsigned d = ok ? ((key[i] >> shift) & mask) : kRadix;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        uint32_t before = 0;
-        if (d < kRadix) before = s_count[warp][d];
+        const bool ok = base + i * 32 < tile_n;
+        const unsigned d = (key[i] >> shift) & mask;
+        if (ok) atomicOr(&s_peers[warp][d], 1u << lane);
         __syncwarp();
-        if (d < kRadix && lane == __ffs(peers) - 1)
-            s_count[warp][d] = before + __popc(peers);
+        const unsigned peers = ok ? s_peers[warp][d] : 0u;
+        const uint32_t before = ok ? s_count[warp][d] : 0u;
         __syncwarp();
-        rank[i] = before + __popc(peers & lt_mask);
+        if (ok && (peers >> lane) == 1u)   // the last of them
+        {
+            s_count[warp][d] = (uint16_t)(before + __popc(peers));
+            s_peers[warp][d] = 0;
+        }
+        __syncwarp();
+        rank[i] = before + __popc(peers & ((1u << lane) - 1u));
     }
     __syncthreads();
-    // Per digit: the tile's count, the warps' starts inside it, and where
-    // the digit's run goes in the output.
-    static_assert(kRadix == kSortThreads, "one digit per thread");
+    // Digit d of the tile: its count, and the warps' starts inside the tile.
+    const int d = threadIdx.x;
+    const unsigned tag = (unsigned)pass + 1u;
+    const unsigned long long tag_bits = (unsigned long long)tag << 40;
+    unsigned long long* col = t.state + d;
+    uint32_t total = 0;
+    if (d < kRadix)
     {
-        const int d = threadIdx.x;
-        uint32_t total = 0;
+#pragma unroll
+        for (int w = 0; w < kSortWarps; ++w) total += s_count[w][d];
+        store_word(col + tile * kRadix,
+                   (tile == 0 ? kTilePrefix : kTileSum) | tag_bits | total);
+    }
+    const uint32_t start = digit_exclusive_scan(total, s_warp);
+    if (d < kRadix)
+    {
+        uint32_t run = start;
 #pragma unroll
         for (int w = 0; w < kSortWarps; ++w)
         {
             const uint32_t c = s_count[w][d];
-            s_count[w][d] = total;   // start of warp w inside the digit
-            total += c;
+            s_count[w][d] = (uint16_t)run;
+            run += c;
         }
-        const uint32_t start = block_exclusive_scan(total, s_warp, &s_total);
-        s_digit_start[d] = start;
-        s_digit_out[d] = offsets[(size_t)d * num_tiles + blockIdx.x];
-#pragma unroll
-        for (int w = 0; w < kSortWarps; ++w) s_count[w][d] += start;
     }
+    // (read only now: eight more registers through the ranking cost a third of
+    // the warps in flight)
+    uint32_t val[kSortItems];
+    const uint32_t* vp = vals_in + tile0 + base;
+#pragma unroll
+    for (int i = 0; i < kSortItems; ++i)
+        val[i] = vals_in && base + i * 32 < tile_n
+                     ? vp[i * 32] : (uint32_t)tile0 + (uint32_t)(base + i * 32);
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < kSortItems; ++i)
-    {
-        const size_t p = base + (size_t)i * 32 + lane;
-        if (p < n)
+        if (base + i * 32 < tile_n)
         {
-            const unsigned d = (key[i] >> shift) & mask;
-            const uint32_t local = s_count[warp][d] + rank[i];
+            const uint32_t local =
+                s_count[warp][(key[i] >> shift) & mask] + rank[i];
             s_keys[local] = key[i];
             s_vals[local] = val[i];
         }
-    }
-    __syncthreads();
-    const int tile_n = (int)min((size_t)kSortTile, n - tile0);
-    for (int q = threadIdx.x; q < tile_n; q += kSortThreads)
+    bool ok = true;
+    if (d < kRadix)
     {
-        const uint32_t k = s_keys[q];
-        const unsigned d = (k >> shift) & mask;
-        const uint32_t dst = s_digit_out[d] + (uint32_t)q - s_digit_start[d];
-        keys_out[dst] = k;
-        vals_out[dst] = s_vals[q];
+        uint32_t before = 0;
+        ok = look_back(col, kRadix, tile, tag, &before);
+        if (ok && tile != 0)
+            store_word(col + tile * kRadix,
+                       kTilePrefix | tag_bits | (before + total));
+        s_out[d] = t.digits[pass * kRadix + d] + before - start;
+    }
+    if (!__syncthreads_and(ok))
+    {
+        if (threadIdx.x == 0)
+            atomicOr(status, (unsigned long long)DEV_ERR_TIMEOUT);
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < kSortItems; ++i)
+    {
+        const int q = i * kSortThreads + threadIdx.x;
+        if (q < tile_n)
+        {
+            const uint32_t k = s_keys[q];
+            const uint32_t dst = s_out[(k >> shift) & mask] + (uint32_t)q;
+            if (dst < n)
+            {
+                keys_out[dst] = k;
+                vals_out[dst] = s_vals[q];
+            }
+        }
     }
 }
-
-
-size_t scan_blocks(size_t n) { return (n + kScanTile - 1) / kScanTile; }
 
 }  // namespace
 
-size_t scan_temp_bytes(size_t n)
-{
-    return (scan_blocks(n) + 1) * sizeof(uint32_t);
-}
-
-cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n,
-                               void* temp, cudaStream_t st, int* launches)
-{
-    if (n == 0) return cudaSuccess;
-    if (launches) *launches += 3;
-    const size_t nb = scan_blocks(n);
-    uint32_t* sums = static_cast<uint32_t*>(temp);
-    scan_reduce_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(in, n, sums);
-    scan_block_sums_kernel<<<1, 1024, 0, st>>>(sums, nb);
-    scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, st>>>(in, out, n, sums);
-    return cudaGetLastError();
-}
-
 size_t radix_sort_temp_bytes(size_t n)
 {
-    const size_t tiles = (n + kSortTile - 1) / kSortTile;
-    const size_t counts = tiles * kRadix;
-    // counts + scanned offsets + scan scratch
-    return 2 * counts * sizeof(uint32_t) + scan_temp_bytes(counts) + 256;
+    return sort_tiles(n) * kRadix * sizeof(unsigned long long) +
+           (kMaxPasses * kRadix + kMaxPasses + 1) * sizeof(uint32_t);
 }
 
 cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
-                             int num_bits, void* temp, cudaStream_t st,
-                             int* which, int* launches)
+                             int num_bits, void* temp,
+                             unsigned long long* status, int num_sms,
+                             cudaStream_t st, int* which, int* launches)
 {
     *which = 0;
-    if (n <= 1 || num_bits <= 0) return cudaSuccess;
-    const size_t tiles = (n + kSortTile - 1) / kSortTile;
-    const size_t ncount = tiles * kRadix;
-    uint32_t* counts = static_cast<uint32_t*>(temp);
-    uint32_t* offsets = counts + ncount;
-    void* scan_tmp = offsets + ncount;
+    if (n == 0) return cudaSuccess;
+    const size_t tiles = sort_tiles(n);
+    const SortTemp t = sort_temp(temp, n);
+    cudaError_t e = cudaMemsetAsync(temp, 0, radix_sort_temp_bytes(n), st);
+    if (e != cudaSuccess) return e;
+    const unsigned cap = (unsigned)num_sms * 4u;
+    const size_t want = (n + 8 * kHistThreads - 1) / (8 * kHistThreads);
+    const unsigned blocks = want < cap ? (unsigned)want : cap;
+    if (num_bits < 1) num_bits = 1;
+    rs_histogram_kernel<<<blocks, kHistThreads, 0, st>>>(keys[0], n, num_bits,
+                                                         t);
+    if (launches) *launches += 1;
     int cur = 0;
-    for (int shift = 0; shift < num_bits; shift += 8)
+    for (int pass = 0; 8 * pass < num_bits; ++pass)
     {
-        const int bits = num_bits - shift < 8 ? num_bits - shift : 8;
-        const uint32_t mask = (1u << bits) - 1u;
-        rs_histogram_kernel<<<(unsigned)tiles, kSortThreads, 0, st>>>(
-            keys[cur], n, shift, mask, tiles, counts);
-        cudaError_t e = exclusive_scan_u32(counts, offsets, ncount, scan_tmp,
-                                           st, launches);
-        if (e != cudaSuccess) return e;
-        rs_scatter_kernel<<<(unsigned)tiles, kSortThreads, 0, st>>>(
-            keys[cur], vals[cur], n, shift, mask, tiles, offsets,
-            keys[cur ^ 1], vals[cur ^ 1]);
-        if (launches) *launches += 2;
+        const int bits = num_bits - 8 * pass < 8 ? num_bits - 8 * pass : 8;
+        rs_pass_kernel<<<(unsigned)tiles, kSortThreads, 0, st>>>(
+            keys[cur], pass ? vals[cur] : nullptr, n, pass, (1u << bits) - 1u,
+            t, status, keys[cur ^ 1], vals[cur ^ 1]);
+        if (launches) *launches += 1;
         cur ^= 1;
     }
     *which = cur;

@@ -130,7 +130,7 @@ extern "C" int oskar_b200_grid_f_static(
     const size_t slab_bytes = static_cube_geometry(P, support, oversample,
                                                    &planes, &max_block,
                                                    &groups);
-    if (!make_key_layout(grid_size, P, 1, &kl, 0, groups))
+    if (!make_key_layout(grid_size, P, 1, num_points, &kl, 0, groups))
         return OSKAR_B200_ERR_UNSUPPORTED;
     const size_t n = num_points;
     const int bpj = prep_blocks_per_job(n, 1, num_sms);
@@ -139,9 +139,11 @@ extern "C" int oskar_b200_grid_f_static(
     int st = scratch_address(device, &base);
     if (st) return st;
     Carver cv{base};
-    auto* counters = cv.take<unsigned long long>(8 * CNT_COUNT);
+    // (counters, skip count, ticket of the prep blocks: what starts from zero)
+    auto* counters = cv.take<unsigned long long>(8 * (CNT_COUNT + 2));
+    unsigned long long* job_skipped = counters + CNT_COUNT;
+    auto* job_ticket = reinterpret_cast<uint32_t*>(job_skipped + 1);
     auto* d_job = cv.take<JobDesc>(sizeof(JobDesc));
-    auto* job_skipped = cv.take<unsigned long long>(8);
     auto* d_planes = cv.take<PlaneDesc>(sizeof(PlaneDesc) * P);
     auto* d_support = cv.take<int>(sizeof(int) * P);
     auto* d_norm_table = cv.take<double>(sizeof(double) * P * span * span);
@@ -150,13 +152,11 @@ extern "C" int oskar_b200_grid_f_static(
     auto* slabs = cv.take<float2>(slab_bytes);
     uint32_t* keys[2] = {cv.take<uint32_t>(4 * n), cv.take<uint32_t>(4 * n)};
     uint32_t* vals[2] = {cv.take<uint32_t>(4 * n), cv.take<uint32_t>(4 * n)};
-    auto* rec = cv.take<int4>(16 * n);
-    auto* tile_counts = cv.take<uint32_t>(8 * task_tiles(n));
+    auto* rec = cv.take<uint2>(sizeof(uint2) * n);
+    auto* task_state = cv.take<unsigned long long>(8 * task_tiles(n));
     auto* task_start = cv.take<uint32_t>(4 * (n + 2));
     auto* task_job = cv.take<uint32_t>(4 * (n + 2));
-    const size_t tmp = std::max(radix_sort_temp_bytes(n > 0 ? n : 1),
-                                scan_temp_bytes(n > 0 ? n : 1));
-    void* scan_tmp = cv.take<unsigned char>(tmp);
+    void* sort_tmp = cv.take<unsigned char>(radix_sort_temp_bytes(n));
     if (cv.used > kStaticScratchBytes) return OSKAR_B200_ERR_OVER_BUDGET;
     if (grid_smem_bytes(0, max_block, false) > 227 * 1024)
         return OSKAR_B200_ERR_UNSUPPORTED;
@@ -204,8 +204,8 @@ extern "C" int oskar_b200_grid_f_static(
     B200_S(cudaMemcpyAsync(d_job, &jd, sizeof(JobDesc),
                            cudaMemcpyHostToDevice, s));
     // The array keeps the last call's contents: clear what accumulates.
-    B200_S(cudaMemsetAsync(counters, 0, 8 * CNT_COUNT, s));
-    B200_S(cudaMemsetAsync(job_skipped, 0, 8, s));
+    B200_S(cudaMemsetAsync(counters, 0, 8 * (CNT_COUNT + 2), s));
+    if (n) B200_S(cudaMemsetAsync(task_state, 0, 8 * task_tiles(n), s));
     B200_S(cudaMemsetAsync(plane_counts, 0, 8 * (size_t)P, s));
     st = static_cube_fill(conv_func, P, oversample, conv_size_half, d_planes,
                           slabs, d_norm_table, s);
@@ -220,24 +220,21 @@ extern "C" int oskar_b200_grid_f_static(
     pa.key = kl;
     pa.rec = rec;
     pa.keys = keys[0];
-    pa.vals = vals[0];
     pa.counters = counters;
     pa.job_skipped = job_skipped;
     pa.norm_partials = partials;
     pa.plane_counts = plane_counts;
-    if (n > 0)
-        B200_S(launch_prep(pa, 0, OSKAR_B200_COORDS_F64, s));
-    else
-        B200_S(cudaMemsetAsync(partials, 0, 8 * (size_t)bpj, s));
-    B200_S(launch_finalize_prep(pa, s));
+    pa.job_tickets = job_ticket;
+    B200_S(launch_prep(pa, 0, OSKAR_B200_COORDS_F64, s));
     if (n == 0) return OSKAR_B200_OK;
     int which = 0;
-    B200_S(radix_sort_pairs(keys, vals, n, kl.total_bits + 1, scan_tmp, s,
-                            &which, nullptr));
+    B200_S(radix_sort_pairs(keys, vals, n, kl.total_bits + 1, sort_tmp,
+                            counters + CNT_STATUS, num_sms, s, &which,
+                            nullptr));
     TaskSizes sizes{};
     while ((1 << sizes.log2_max[0]) < kTaskMax) ++sizes.log2_max[0];
     B200_S(launch_tasks(keys[which], n, counters, 2 * kl.fine_bits,
-                        kl.job_shift, sizes, tile_counts, scan_tmp,
+                        kl.job_shift, sizes, task_state,
                         task_start, task_job, s, nullptr));
     GridArgs ga{};
     ga.order = vals[which];

@@ -122,13 +122,12 @@ weights_write_atomic_kernel(size_t n, const T* __restrict__ uu,
 }
 
 // Sort keys for the ordered write: the cell, or `sentinel` (= grid_size^2,
-// above every cell) for a skipped point; values are the point indices.
+// above every cell) for a skipped point.
 template <typename T>
 __global__ void __launch_bounds__(256)
 weights_key_kernel(size_t n, const T* __restrict__ uu,
                    const T* __restrict__ vv, WeightConsts c,
                    uint32_t sentinel, uint32_t* __restrict__ keys,
-                   uint32_t* __restrict__ vals,
                    unsigned long long* __restrict__ skipped)
 {
     unsigned local = 0;
@@ -139,7 +138,6 @@ weights_key_kernel(size_t n, const T* __restrict__ uu,
         const long long t = weight_cell(uu[i], vv[i], c);
         local += t < 0;
         keys[i] = t < 0 ? sentinel : (uint32_t)t;
-        vals[i] = (uint32_t)i;
     }
     count_skipped(local, skipped);
 }
@@ -157,8 +155,15 @@ __global__ void __launch_bounds__(256)
 weights_run_sum_kernel(size_t n, const uint32_t* __restrict__ keys,
                        const uint32_t* __restrict__ vals,
                        const T* __restrict__ weight, uint32_t sentinel,
-                       T* __restrict__ grid)
+                       T* __restrict__ grid,
+                       const unsigned long long* __restrict__ status,
+                       unsigned long long* __restrict__ skipped)
 {
+    if (*status)   // the sort gave up: its pairs are not to be used
+    {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *skipped = kSortFailed;
+        return;
+    }
     const int lane = threadIdx.x & 31;
     const size_t warp0 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const size_t warps = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -337,7 +342,10 @@ int run_weights_write(oskar_B200Workspace* ws, int data_is_double,
     B200_TRY(ws->keys[1].ensure(4 * n));
     B200_TRY(ws->vals[0].ensure(4 * n));
     B200_TRY(ws->vals[1].ensure(4 * n));
-    B200_TRY(ws->scan_tmp.ensure(radix_sort_temp_bytes(n)));
+    B200_TRY(ws->sort_tmp.ensure(radix_sort_temp_bytes(n)));
+    unsigned long long* status =
+        static_cast<unsigned long long*>(ws->counters.ptr) + CNT_STATUS;
+    B200_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned long long), st));
     uint32_t* keys[2] = {static_cast<uint32_t*>(ws->keys[0].ptr),
                          static_cast<uint32_t*>(ws->keys[1].ptr)};
     uint32_t* vals[2] = {static_cast<uint32_t*>(ws->vals[0].ptr),
@@ -348,24 +356,25 @@ int run_weights_write(oskar_B200Workspace* ws, int data_is_double,
     if (data_is_double)
         weights_key_kernel<double><<<blocks, 256, 0, st>>>(
             n, (const double*)uu, (const double*)vv, c, sentinel, keys[0],
-            vals[0], skipped);
+            skipped);
     else
         weights_key_kernel<float><<<blocks, 256, 0, st>>>(
             n, (const float*)uu, (const float*)vv, c, sentinel, keys[0],
-            vals[0], skipped);
+            skipped);
     B200_TRY(cudaGetLastError());
     ++launches;
     int which = 0;
     B200_TRY(radix_sort_pairs(keys, vals, n, bit_length(cells),
-                              ws->scan_tmp.ptr, st, &which, &launches));
+                              ws->sort_tmp.ptr, status, ws->num_sms, st,
+                              &which, &launches));
     if (data_is_double)
         weights_run_sum_kernel<double><<<blocks, 256, 0, st>>>(
             n, keys[which], vals[which], (const double*)weight, sentinel,
-            (double*)grid);
+            (double*)grid, status, skipped);
     else
         weights_run_sum_kernel<float><<<blocks, 256, 0, st>>>(
             n, keys[which], vals[which], (const float*)weight, sentinel,
-            (float*)grid);
+            (float*)grid, status, skipped);
     B200_TRY(cudaGetLastError());
     ++launches;
     ws->last_launches = launches;
