@@ -57,14 +57,12 @@ struct __align__(16) TapVis
     typename Vec2<GT>::type c0, c1;
 };
 
-// A task's visibility as gathered from the caller's order: its placement
-// record and its visibility (times its weight when asked for).  The task's
-// raw records occupy the start of the tap-record array until derive() has
-// read them.
+// A visibility as gathered from the caller's order: its placement record and
+// its visibility (times its weight when asked for).
 template <typename GT>
-struct __align__(16) RawVis
+struct RawVis
 {
-    int4 rec;
+    uint2 rec;
     typename Vec2<GT>::type vis;
 };
 
@@ -274,18 +272,6 @@ __device__ __forceinline__ uint32_t task_order(uint32_t key,
         }
     }
     return key;
-}
-
-// Two records that read the same kernel values into the same cells.  Their
-// contributions are vis_a * Kt + vis_b * Kt = (vis_a + vis_b) * Kt: the tap
-// coefficients (which fold in the conjugation) can simply be added.
-template <typename GT>
-__device__ __forceinline__ bool same_taps(const TapVis<GT>& a,
-                                          const TapVis<GT>& b)
-{
-    return a.origin == b.origin && a.mu == b.mu && a.mv == b.mv &&
-           a.tu == b.tu && a.cp == b.cp && a.cn == b.cn &&
-           a.base == b.base;
 }
 
 // Predicated complex flush: one vector reduction when `pred` holds, no
@@ -587,15 +573,31 @@ romein_grid_kernel(const GridArgs a)
 {
     using V2 = typename Vec2<GT>::type;
     extern __shared__ __align__(128) unsigned char smem[];
-    // STAGED: [row block of the current run][tap records]; else [records]
+    // [row block of the current run (STAGED)][tap records]
     KT* s_block = reinterpret_cast<KT*>(smem);
     TapVis<GT>* s_vis = reinterpret_cast<TapVis<GT>*>(
         smem + (STAGED ? a.block_smem_bytes : 0));
+    // A batch's raw points lie at the end of the tap records, behind the
+    // first kKeep (a place of their own cost 4 KB of L1 per CTA, 8 in FP64).
+    constexpr int kKeep = kTaskMax - (int)((kTaskMax * sizeof(RawVis<GT>) +
+                                            sizeof(TapVis<GT>) - 1) /
+                                           sizeof(TapVis<GT>));
+    RawVis<GT>* s_raw = reinterpret_cast<RawVis<GT>*>(s_vis + kKeep);
     __shared__ uint64_t s_bar;
-    __shared__ unsigned long long s_task;
+    // The CTA's task: what is left of it when the classes run (kept here and
+    // not in registers, which the tap loop needs).
+    __shared__ struct
+    {
+        const JobDesc* job;
+        uint32_t begin;   // its first sorted position
+        int total;        // its points; -1: no task is left
+        int done;         // points gathered
+        int pending;      // merged points of the batch in s_raw
+        uint2 point;      // record of one of its points
+    } s_task;
     __shared__ uint32_t s_order[kGridThreads];
     __shared__ int s_run_begin[kMaxOffsets], s_run_end[kMaxOffsets];
-    __shared__ unsigned char s_head[kTaskMax];
+    __shared__ bool s_head[kTaskMax + 1];
     __shared__ int4 s_box[kGridThreads / 32];
     __shared__ int s_warp_heads[kGridThreads / 32];
 
@@ -619,158 +621,204 @@ romein_grid_kernel(const GridArgs a)
 
     uint32_t phase = 0;
     unsigned flushes = 0;
+    const int t = threadIdx.x;
+    if (t == 0) s_task.total = s_task.done = s_task.pending = 0;
     for (;;)
     {
-        if (threadIdx.x == 0) s_task = first + atomicAdd(queue, 1ull);
-        if (threadIdx.x < kMaxOffsets)
-        {
-            s_run_begin[threadIdx.x] = 0;
-            s_run_end[threadIdx.x] = 0;
-        }
-        // Also: every thread has finished with the previous task's records
-        // and row block before they are overwritten below.
+        // Every thread has finished with the records, the row block and the
+        // task before they are overwritten below.
         __syncthreads();
-        if (s_task >= end) break;
-        const unsigned task = (unsigned)s_task;
-        const uint32_t begin = a.task_start[task];
-        int m = (int)(a.task_start[task + 1] - begin);
-        if (m <= 0 || m > kTaskMax)
+        if (t == 0 && s_task.pending == 0 && s_task.done == s_task.total)
         {
-            if (threadIdx.x == 0)
-                atomicOr(status, (unsigned long long)DEV_ERR_TASK);
-            __syncthreads();   // s_task is read before thread 0 rewrites it
-            continue;
-        }
-        // The task's job: its cube, grid and geometry.
-        const JobDesc& jd = a.jobs[a.task_job[task]];
-        const int t = threadIdx.x;
-        // Gather the task's visibilities (sorted positions begin .. begin +
-        // m - 1) straight from the caller's arrays: record, visibility and
-        // weight of each point.  Against a separate pass that permuted
-        // records and visibilities into sorted order: plain_large step
-        // 19.15 -> 18.25 ms (the 1.6 ms pass gone, the gridding kernel
-        // 0.7 ms slower with the gathers in its task set-up; prefetching
-        // the next task's points into L2 cost more than it hid).
-        static_assert(sizeof(RawVis<GT>) <= sizeof(TapVis<GT>),
-                      "raw records fit the tap-record array");
-        RawVis<GT>* s_raw = reinterpret_cast<RawVis<GT>*>(s_vis);
-        uint32_t key = 0xffffffffu;
-        int4 myrec = make_int4(0, 0, 0, 0);
-        if (t < m)
-        {
-            const uint32_t i = a.order[begin + t];
-            RawVis<GT> rv;
-            rv.rec = unpack_record(a.rec[i]);
-            const size_t local = i - jd.first;
-            const GT* __restrict__ vis = static_cast<const GT*>(jd.vis);
-            GT re = vis[2 * local], im = vis[2 * local + 1];
-            if (a.apply_weight)
+            const unsigned long long task = first + atomicAdd(queue, 1ull);
+            s_task.done = 0;
+            if (task >= end)
+                s_task.total = -1;
+            else
             {
-                const GT wt = static_cast<const GT*>(jd.weight)[local];
-                re *= wt;
-                im *= wt;
+                const uint32_t begin = a.task_start[task];
+                const int total = (int)(a.task_start[task + 1] - begin);
+                s_task.begin = begin;
+                s_task.job = a.jobs + a.task_job[task];
+                s_task.total = total;
+                if (total <= 0 || total > (STAGED ? kTaskMax : kTaskRaw))
+                {
+                    atomicOr(status, (unsigned long long)DEV_ERR_TASK);
+                    s_task.total = 0;
+                }
             }
-            rv.vis.x = re;
-            rv.vis.y = im;
-            s_raw[t] = rv;
-            myrec = rv.rec;
         }
-        const TaskKey tk(jd.half, task_box(t < m, myrec, s_box));
-        if (t < m) key = tk.template make<!STAGED>(myrec, t);
-        // Order the task's visibilities (see TaskKey): consecutive ones are
-        // neighbours.  (Its block barriers also publish the raw records.)
-        static_assert(kGridThreads >= 64, "task_order has a block barrier");
-        key = task_order(key, s_order);
-        const KT* __restrict__ slabs = static_cast<const KT*>(jd.slabs);
-        const int4 r0 = s_raw[0].rec;
-        // Compensation is limited to tasks near the grid centre when a
-        // radius is set (a task is a compact run of one coarse tile).
-        bool comp_here = true;
-        if (COMP && a.comp_radius > 0)
+        if (t < kMaxOffsets)
         {
-            const int c = jd.grid_size / 2;
-            comp_here = abs(r0.x - c) <= a.comp_radius &&
-                        abs(r0.y - c) <= a.comp_radius;
+            s_run_begin[t] = 0;
+            s_run_end[t] = 0;
         }
-        const auto fl = make_flush<GT, COMP>(jd, a.comp_part, comp_here);
-        const int grid_size = jd.grid_size;
-        const int offsets = 2 * jd.half + 1;
-        const int plane = r0.z & 0x7fffffff;
+        __syncthreads();
+        const int total = s_task.total;
+        if (total < 0) break;
+        if (total == 0) continue;
+        // The task's job: its cube, grid and geometry.
+        const JobDesc& jd = *s_task.job;
+        const uint32_t begin = s_task.begin;
+        const KT* __restrict__ slabs = static_cast<const KT*>(jd.slabs);
         const PlaneDesc* __restrict__ planes = jd.planes;
-        const PlaneDesc d = planes[plane];
-        const int w = 2 * d.support + 1;
+        const int grid_size = jd.grid_size;
+        // The task's points come in batches of at most kTaskMax.  A batch is
+        // ordered, its points with identical placements are merged, and the
+        // merged ones are appended to the tap records; the classes run when
+        // the next batch does not fit any more.  Where many points share
+        // their placement (dense cells near the uv origin) one run then
+        // serves several batches: a quarter of the flushes into the densest
+        // cells, whose FP32 sums are rounded that much less often (2.2 M
+        // points on 3000^2: error against FP64 1.5e-6 -> 0.65e-6, gridding
+        // 518 -> 508 us; one batch per task was 1 % faster on 39.2 M points,
+        // 3 % on 24 channels).
+        int done = s_task.done, pending = s_task.pending;
+        int count = 0;     // tap records
+        for (;;)
+        {
+            if (pending == 0)
+            {
+                if (done == total || count > kKeep) break;
+                // Gather the batch (sorted positions begin + done ...)
+                // straight from the caller's arrays: record, visibility
+                // and weight of each point.  Against a separate pass that
+                // permuted records and visibilities into sorted order:
+                // plain_large step 19.15 -> 18.25 ms (the 1.6 ms pass
+                // gone, the gridding kernel 0.7 ms slower; prefetching
+                // the next task's points into L2 cost more than it hid).
+                const int m = min(total - done, kTaskMax);
+                int4 rec = make_int4(0, 0, 0, 0);
+                if (t < m)
+                {
+                    const uint32_t i = a.order[begin + done + t];
+                    RawVis<GT> rv;
+                    rv.rec = a.rec[i];
+                    const size_t local = i - jd.first;
+                    const GT* __restrict__ vis =
+                        static_cast<const GT*>(jd.vis);
+                    GT re = vis[2 * local], im = vis[2 * local + 1];
+                    if (a.apply_weight)
+                    {
+                        const GT wt =
+                            static_cast<const GT*>(jd.weight)[local];
+                        re *= wt;
+                        im *= wt;
+                    }
+                    rv.vis.x = re;
+                    rv.vis.y = im;
+                    s_raw[t] = rv;
+                    if (t == 0) s_task.point = rv.rec;
+                    rec = unpack_record(rv.rec);
+                }
+                const TaskKey tk(jd.half, task_box(t < m, rec, s_box));
+                uint32_t key = 0xffffffffu;
+                if (t < m) key = tk.template make<!STAGED>(rec, t);
+                // Order the batch (see TaskKey): consecutive points are
+                // neighbours.  (Its block barriers also publish the raw
+                // records.)
+                static_assert(kGridThreads >= 64,
+                              "task_order has a block barrier");
+                key = task_order(key, s_order);
+                s_order[t] = key;
+                __syncthreads();
+                // Points with the same record read the same kernel values
+                // into the same cells: the first of each run stands for
+                // it with the sum of their visibilities.
+                bool head = false;
+                if (t < m)
+                {
+                    const uint2 r = s_raw[key & 0xffu].rec;
+                    const uint2 q =
+                        s_raw[s_order[t ? t - 1 : 0] & 0xffu].rec;
+                    head = t == 0 || r.x != q.x || r.y != q.y;
+                }
+                // (the end of the batch ends its last run)
+                s_head[t] = head || t >= m;
+                if (t == 0) s_head[kTaskMax] = true;
+                const unsigned ball = __ballot_sync(0xffffffffu, head);
+                if ((t & 31) == 0) s_warp_heads[t >> 5] = __popc(ball);
+                __syncthreads();
+                for (int wi = 0; wi < kGridThreads / 32; ++wi)
+                    pending += s_warp_heads[wi];
+                done += m;
+            }
+            if (count + pending > kTaskMax) break;
+            // Append the batch's merged points.
+            const int batch = done - (done - 1) / kTaskMax * kTaskMax;
+            const bool head = t < batch && s_head[t];
+            const unsigned ball = __ballot_sync(0xffffffffu, head);
+            int pos = count + __popc(ball & ((1u << (t & 31)) - 1u));
+            for (int wi = 0; wi < (t >> 5); ++wi) pos += s_warp_heads[wi];
+            TapVis<GT> tv;
+            if (head)
+            {
+                RawVis<GT> rv = s_raw[s_order[t] & 0xffu];
+                for (int q = t + 1; !s_head[q]; ++q)
+                {
+                    const RawVis<GT>& o = s_raw[s_order[q] & 0xffu];
+                    rv.vis.x += o.vis.x;
+                    rv.vis.y += o.vis.y;
+                }
+                const int4 rec = unpack_record(rv.rec);
+                tv = derive<GT, KT>(rec, rv.vis,
+                                    planes[rec.z & 0x7fffffff],
+                                    STAGED ? nullptr : slabs, grid_size,
+                                    jd.oversample, jd.half, status);
+            }
+            const uint32_t key = s_order[t];
+            __syncthreads();   // the raw batch is read
+            if (head) s_vis[pos] = tv;
+            if (STAGED)
+            {
+                // The runs of each row offset in the merged order.
+                if (head) s_order[pos] = key;
+                __syncthreads();
+                if (t < pending)
+                {
+                    const TaskKey tk(jd.half, make_int4(0, 0, 0, 0));
+                    const int ov = tk.row_offset(s_order[t]);
+                    if (t == 0 || tk.row_offset(s_order[t - 1]) != ov)
+                        s_run_begin[ov] = t;
+                    if (t == pending - 1 ||
+                        tk.row_offset(s_order[t + 1]) != ov)
+                        s_run_end[ov] = t + 1;
+                }
+            }
+            __syncthreads();
+            count += pending;
+            pending = 0;
+        }
+        // Any point of the task tells its geometry (its planes share it).
+        const uint2 r0 = s_task.point;
+        const PlaneDesc d = planes[r0.y & 0x7fffu];
+        const int w = 2 * d.support + 1, offsets = 2 * jd.half + 1;
+        if (t == 0)
+        {
+            s_task.done = done;
+            s_task.pending = pending;
+        }
         // No kept footprint is wider than its grid; a task that says
         // otherwise is malformed (and its cells could leave the grid).
         if (w > grid_size)
         {
-            if (threadIdx.x == 0)
-                atomicOr(status, (unsigned long long)DEV_ERR_TASK);
-            __syncthreads();   // s_task is read before thread 0 rewrites it
+            if (t == 0) atomicOr(status, (unsigned long long)DEV_ERR_TASK);
             continue;
         }
         const int cpt = d.support < kTuneMax ? a.cpt[d.support] : 5;
-
-        RawVis<GT> mine;
-        if (t < m) mine = s_raw[key & 0xffu];
-        __syncthreads();   // every raw record is read before it is overwritten
-        TapVis<GT> tv;
-        if (t < m)
+        // Compensation is limited to tasks near the grid centre when a radius
+        // is set (a task is a compact run of one coarse tile).
+        bool comp_here = true;
+        if (COMP && a.comp_radius > 0)
         {
-            tv = derive<GT, KT>(mine.rec, mine.vis,
-                                planes[mine.rec.z & 0x7fffffff],
-                                STAGED ? nullptr : slabs, grid_size,
-                                jd.oversample, jd.half, status);
-            s_vis[t] = tv;
+            const int c = grid_size / 2;
+            comp_here = abs((int)(r0.x & 0xffffu) - c) <= a.comp_radius &&
+                        abs((int)(r0.x >> 16) - c) <= a.comp_radius;
         }
-        __syncthreads();
-        // Merge runs of records with the same taps (the same cell, plane
-        // and offsets: adjacent in this order): their coefficients add.
-        // Dense cells hold many visibilities with identical placements; at
-        // plain_large this removes a sixth of the taps.
-        const bool head = t < m && (t == 0 || !same_taps(tv, s_vis[t - 1]));
-        s_head[t] = head ? 1 : 0;
-        const unsigned ball = __ballot_sync(0xffffffffu, head);
-        if ((t & 31) == 0) s_warp_heads[t >> 5] = __popc(ball);
-        __syncthreads();
-        int pos = __popc(ball & ((1u << (t & 31)) - 1u)), merged = 0;
-#pragma unroll
-        for (int wi = 0; wi < kGridThreads / 32; ++wi)
-        {
-            pos += wi < (t >> 5) ? s_warp_heads[wi] : 0;
-            merged += s_warp_heads[wi];
-        }
-        if (head)
-        {
-            for (int q = t + 1; q < m && !s_head[q]; ++q)
-            {
-                tv.c0.x += s_vis[q].c0.x;
-                tv.c0.y += s_vis[q].c0.y;
-                tv.c1.x += s_vis[q].c1.x;
-                tv.c1.y += s_vis[q].c1.y;
-            }
-        }
-        __syncthreads();   // every run has been read
-        if (head)
-        {
-            s_vis[pos] = tv;
-            s_order[pos] = key;
-        }
-        __syncthreads();
-        m = merged;
-        if (STAGED && t < m)
-        {
-            key = s_order[t];
-            const int ov = tk.row_offset(key);
-            if (t == 0 || tk.row_offset(s_order[t - 1]) != ov)
-                s_run_begin[ov] = t;
-            if (t == m - 1 || tk.row_offset(s_order[t + 1]) != ov)
-                s_run_end[ov] = t + 1;
-        }
-        __syncthreads();
-
+        const auto fl = make_flush<GT, COMP>(jd, a.comp_part, comp_here);
         if (!STAGED)
         {
-            dispatch_cpt<GT, KT, COUNT, true>(cpt, s_vis, m, w, d.pitch, 0,
+            dispatch_cpt<GT, KT, COUNT, true>(cpt, s_vis, count, w, d.pitch, 0,
                                         slabs, fl, grid_size, flushes);
             continue;
         }

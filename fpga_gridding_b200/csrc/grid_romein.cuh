@@ -11,7 +11,8 @@ constexpr int kGridThreads = 256;   // threads per CTA
 // coefficients are twice as wide and spill at 64).
 template <typename GT>
 constexpr int grid_ctas_per_sm() { return sizeof(GT) == 8 ? 3 : 4; }
-constexpr int kTaskMax = 256;       // visibilities per task
+constexpr int kTaskMax = 256;       // tap records (merged points) at a time
+constexpr int kTaskRaw = 1024;      // points per task (staged: kTaskMax)
 constexpr int kTuneMax = 128;       // supports covered by the tune table
 constexpr unsigned kBulkChunk = 32768;  // bytes per cp.async.bulk
 constexpr int kMaxOffsets = 33;     // 2 * ceil(oversample / 2) + 1, oversample <= 32

@@ -262,7 +262,7 @@ bool make_key_layout(int grid_size, int num_planes, int num_jobs,
 // Sets each plane's group and returns the groups' supports (ascending, at
 // most 128: supports are <= 127).
 std::vector<int> assign_groups(PlaneDesc* planes, int num_planes);
-// Points per task of each group, as powers of two (at most kTaskMax).
+// Points per task of each group, as powers of two (at most kTaskRaw).
 struct TaskSizes
 {
     uint32_t group_mask;           // of the group field; 0: log2_max[0] for all

@@ -85,7 +85,11 @@ double coord_scale_of(double frequency_hz)
 // launch leave the device idle: wide groups get smaller tasks, to at most
 // `cap` taps, the smaller the fewer points the launch has to fill the
 // device with.  Smaller tasks merge and share less and repeat their set-up.
-// Gridding time without a cap and with caps of 4e5, 2e5, 1e5, 5e4 taps:
+// Up to kTaskRaw points, whose merged batches share a run of the classes, or,
+// in jobs too small to fill the device with such tasks, one batch (10 thousand
+// points: 16.4 against 18.5 us).
+// Gridding time without a cap and with caps of 4e5, 2e5, 1e5, 5e4 taps (tasks
+// of one batch):
 //   39.2 M points on 8192^2    16.28, 16.29, 16.55, 17.35, 18.92 ms
 //   2.2 M points on 3000^2      551, 553, 525, 519, 557 us
 //   0.24 M points on 1024^2      49, 51, 47, 46, 53 us
@@ -96,7 +100,8 @@ static TaskSizes task_sizes(const KeyLayout& kl, int num_jobs,
 {
     TaskSizes t{};
     int full = 0;
-    while ((1 << full) < kTaskMax) ++full;
+    const bool batches = !kl.by_plane && points > (size_t(1) << 16);
+    while ((1 << full) < (batches ? kTaskRaw : kTaskMax)) ++full;
     if (kl.by_plane)
     {
         t.log2_max[0] = (unsigned char)full;

@@ -13,18 +13,18 @@
 namespace b200 {
 
 // Sort key bits (skip flag included) that the fine cell index may fill: whole
-// passes of the sort, enough to tell about four times as many places apart as
-// there are points.  More bits cost a pass; fewer put points of a wider block
-// into a task in arrival order, which its own sort cannot undo.  One B200, 32
-// -> 24 bits: 2.2 M points, sort 136 -> 108 us, gridding 516 -> 533; 3.4 M
-// 161 -> 124, 5070 -> 5074; 39.2 M 1361 -> 1039, 16199 -> 18779.  24 -> 16:
-// 10 thousand points, sort 38 -> 30 us, gridding 16.4 both; 0.24 M 46 -> 32,
-// 45 -> 68.
+// passes of the sort.  Fewer bits put points of a wider block into a task in
+// arrival order, which its own sort cannot undo: its columns are then swept
+// again and again, and the densest cells take more roundings.  One B200, 16 /
+// 24 / 32 bits: 10 thousand points, sort 30 / 38 / 38 us, gridding 16 us each;
+// 0.24 M, 32 / 46 / 57 and 68 / 45 / 45 us; 2.2 M, 77 / 108 / 136 and 703 /
+// 541 / 508 us, error against FP64 1.5e-6 with 24 bits, 0.65e-6 with 32;
+// 39.2 M, 0.70 / 1.04 / 1.36 and 29.4 / 18.8 / 16.2 ms.
 static int key_bits(size_t num_points)
 {
-    int b = 2;
-    while ((size_t(1) << (b - 2)) < num_points && b < 32) ++b;
-    return std::min(32, (b + 7) / 8 * 8);
+    return num_points <= (size_t(1) << 14)   ? 16
+           : num_points <= (size_t(1) << 18) ? 24
+                                             : 32;
 }
 
 std::vector<int> assign_groups(PlaneDesc* planes, int num_planes)

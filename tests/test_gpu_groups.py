@@ -49,7 +49,21 @@ def _job(name, oversample, spread, n=3000, grid=500):
 def test_groups_match_oracle(oracle, name, oversample, spread, single, accum):
     if accum == _lib.ACCUM_COMPENSATED and not single:
         pytest.skip("compensated accumulation is FP32 only")
-    w = _job(name, oversample, spread)
+    _check(oracle, _job(name, oversample, spread), oversample, single, accum)
+
+
+@pytest.mark.parametrize("single,accum", [
+    (False, _lib.ACCUM_PLAIN), (True, _lib.ACCUM_PLAIN),
+    (True, _lib.ACCUM_COMPENSATED)])
+@pytest.mark.parametrize("spread", [1.5, 6.0, 205.0])
+@pytest.mark.parametrize("name", ["constant", "mixed", "one"])
+def test_batches_match_oracle(oracle, name, spread, single, accum):
+    """Enough points that a task holds several batches: all merged into a few
+    records, some, none."""
+    _check(oracle, _job(name, 4, spread, n=80000), 4, single, accum)
+
+
+def _check(oracle, w, oversample, single, accum):
     real = np.float32 if single else np.float64
     ref = dict(w)
     for k in ("conv_func", "uu", "vv", "ww", "vis", "weight"):
