@@ -213,15 +213,17 @@ enum CounterSlot
 
 // ---- radix_sort.cu --------------------------------------------------------
 size_t radix_sort_temp_bytes(size_t n);
-// Stable LSD sort of (key, position) pairs on the low num_bits of the keys in
-// keys[0]; the values are the positions 0 .. n - 1.  The sorted pairs end in
+// Stable LSD sort of (key, value) pairs on the low num_bits of the keys in
+// keys[0]; the values are first_vals, which is only read, or the positions
+// 0 .. n - 1 where that is null.  The sorted pairs end in
 // keys[*which] / vals[*which].  *status: the device status word; when it has
 // DEV_ERR_TIMEOUT (set here when a bounded wait expires) the pairs are not to
 // be used.
 cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
                              int num_bits, void* temp,
                              unsigned long long* status, int num_sms,
-                             cudaStream_t st, int* which, int* launches);
+                             cudaStream_t st, int* which, int* launches,
+                             const uint32_t* first_vals = nullptr);
 
 // ---- cube.cu ----------------------------------------------------------------
 // d_conv_im == nullptr: d_conv_func is the interleaved complex cube;

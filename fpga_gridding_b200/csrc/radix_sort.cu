@@ -343,7 +343,8 @@ size_t radix_sort_temp_bytes(size_t n)
 cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
                              int num_bits, void* temp,
                              unsigned long long* status, int num_sms,
-                             cudaStream_t st, int* which, int* launches)
+                             cudaStream_t st, int* which, int* launches,
+                             const uint32_t* first_vals)
 {
     *which = 0;
     if (n == 0) return cudaSuccess;
@@ -363,7 +364,7 @@ cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
     {
         const int bits = num_bits - 8 * pass < 8 ? num_bits - 8 * pass : 8;
         rs_pass_kernel<<<(unsigned)tiles, kSortThreads, 0, st>>>(
-            keys[cur], pass ? vals[cur] : nullptr, n, pass, (1u << bits) - 1u,
+            keys[cur], pass ? vals[cur] : first_vals, n, pass, (1u << bits) - 1u,
             t, status, keys[cur ^ 1], vals[cur ^ 1]);
         if (launches) *launches += 1;
         cur ^= 1;
