@@ -577,7 +577,7 @@ size_t oskar_b200_workspace_bytes(const oskar_B200Workspace* ws)
     if (!ws) return 0;
     const DeviceBuffer* bufs[] = {
         &ws->keys[0], &ws->keys[1], &ws->vals[0], &ws->vals[1], &ws->rec,
-        &ws->sort_tmp, &ws->task_start, &ws->task_job,
+        &ws->task_start, &ws->task_job,
         &ws->counters, &ws->partials, &ws->in_uu,
         &ws->in_vv, &ws->in_ww, &ws->in_vis, &ws->in_weight, &ws->in_grid,
         &ws->in_cube, &ws->in_norm, &ws->comp_grid};

@@ -126,7 +126,7 @@ struct oskar_B200Workspace
     size_t smem_optin = 0;
     cudaStream_t stream = nullptr;
     // per-visibility work arrays
-    b200::DeviceBuffer keys[2], vals[2], rec, sort_tmp;
+    b200::DeviceBuffer keys[2], vals[2], rec;
     b200::DeviceBuffer task_start, task_job;
     // small arrays: what a call starts from zero (the counters first, then
     // see run_batch), partial sums, the job table
@@ -218,7 +218,7 @@ size_t radix_sort_temp_bytes(size_t n);
 // 0 .. n - 1 where that is null.  The sorted pairs end in
 // keys[*which] / vals[*which].  *status: the device status word; when it has
 // DEV_ERR_TIMEOUT (set here when a bounded wait expires) the pairs are not to
-// be used.
+// be used.  temp: radix_sort_temp_bytes(n) zeroed bytes.
 cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
                              int num_bits, void* temp,
                              unsigned long long* status, int num_sms,

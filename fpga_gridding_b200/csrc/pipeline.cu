@@ -208,7 +208,8 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     B200_TRY(cudaStreamIsCapturing(st, &capture));
     const bool capturing = capture != cudaStreamCaptureStatusNone;
-    // The job table goes up from the next pinned buffer of the ring; the
+    // One job goes to prep with its arguments, and prep writes the table.  The
+    // table of several goes up from the next pinned buffer of the ring; the
     // upload that last read that buffer must have happened before it is
     // rewritten.  (A caller capturing a graph has synchronised.)
     // Every buffer of the ring is (re)allocated together, so that a call
@@ -235,10 +236,13 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         }
     }
     const int slot = ws->jobs_slot;
-    ws->jobs_slot = (slot + 1) % kJobRing;
-    if (ws->jobs_event_pending[slot] && !capturing)
-        B200_TRY(cudaEventSynchronize(ws->jobs_event[slot]));
-    ws->jobs_event_pending[slot] = 0;
+    if (num_jobs > 1)
+    {
+        ws->jobs_slot = (slot + 1) % kJobRing;
+        if (ws->jobs_event_pending[slot] && !capturing)
+            B200_TRY(cudaEventSynchronize(ws->jobs_event[slot]));
+        ws->jobs_event_pending[slot] = 0;
+    }
     // FP64 sums of the real and of the imaginary parts.  Where there is no
     // room for both, the tasks run twice and share one plane of sums.
     int comp_passes = comp ? 1 : 0;
@@ -248,7 +252,9 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         comp_passes = 2;
         B200_TRY(ws->comp_grid.ensure(comp_cells * sizeof(double)));
     }
-    JobDesc* hj = static_cast<JobDesc*>(ws->h_jobs[slot]);
+    PrepArgs pa{};
+    JobDesc* hj = num_jobs == 1 ? &pa.job
+                                : static_cast<JobDesc*>(ws->h_jobs[slot]);
     size_t first = 0, comp_off = 0;
     for (int j = 0; j < num_jobs; ++j)
     {
@@ -294,11 +300,13 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     // What starts from zero, in one buffer and one memset: the counters, then
     // per job the skip count, the plane histogram and the ticket of its prep
     // blocks (a word each, of which half is used), then the task list's tile
-    // words.
+    // words and the sort's scratch.
     const size_t zero_words = CNT_COUNT +
                               (size_t)num_jobs * (2 + (size_t)max_planes) +
                               task_tiles(n);
-    B200_TRY(ws->counters.ensure(sizeof(unsigned long long) * zero_words));
+    const size_t zero_bytes = sizeof(unsigned long long) * zero_words +
+                              (n ? radix_sort_temp_bytes(n) : 0);
+    B200_TRY(ws->counters.ensure(zero_bytes));
     B200_TRY(ws->jobs.ensure(job_bytes));
     B200_TRY(ws->partials.ensure(sizeof(double) * num_jobs * bpj));
     unsigned long long* counters =
@@ -308,11 +316,16 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     unsigned long long* job_tickets =
         plane_counts + (size_t)num_jobs * max_planes;
     unsigned long long* task_state = job_tickets + num_jobs;
-    B200_TRY(cudaMemsetAsync(counters, 0,
-                             sizeof(unsigned long long) * zero_words, st));
-    B200_TRY(cudaMemcpyAsync(ws->jobs.ptr, hj, job_bytes,
-                             cudaMemcpyHostToDevice, st));
+    void* sort_temp = counters + zero_words;
+    B200_TRY(cudaMemsetAsync(counters, 0, zero_bytes, st));
+    if (num_jobs == 1)
     {
+        pa.job_out = static_cast<JobDesc*>(ws->jobs.ptr);
+    }
+    else
+    {
+        B200_TRY(cudaMemcpyAsync(ws->jobs.ptr, hj, job_bytes,
+                                 cudaMemcpyHostToDevice, st));
         // Outside stream capture, remember when the upload has happened.
         if (!capturing)
         {
@@ -337,10 +350,8 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
             B200_TRY(ws->task_start.ensure(4 * (n + 2)));
             B200_TRY(ws->task_job.ensure(4 * (n + 2)));
         }
-        B200_TRY(ws->sort_tmp.ensure(radix_sort_temp_bytes(n)));
     }
 
-    PrepArgs pa{};
     pa.jobs = d_jobs;
     pa.num_jobs = num_jobs;
     pa.blocks_per_job = bpj;
@@ -381,7 +392,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
 
     int which = 0;
     B200_TRY(radix_sort_pairs(keys, vals, n, kl.total_bits + 1,
-                              ws->sort_tmp.ptr, counters + CNT_STATUS,
+                              sort_temp, counters + CNT_STATUS,
                               ws->num_sms, st, &which, &launches));
     B200_TRY(mark(2));
     if (degrid)

@@ -137,10 +137,15 @@ __device__ __forceinline__ PlaceConsts place_consts(const JobDesc& jd)
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kPrepThreads)
-prep_kernel(const PrepArgs a)
+prep_kernel(const __grid_constant__ PrepArgs a)
 {
     const int job = blockIdx.y;
-    const JobDesc& jd = a.jobs[job];
+    const JobDesc& jd = a.job_out ? a.job : a.jobs[job];
+    static_assert(sizeof(JobDesc) % 4 == 0 &&
+                  sizeof(JobDesc) / 4 <= kPrepThreads, "a word per thread");
+    if (a.job_out && blockIdx.x == 0 && threadIdx.x < sizeof(JobDesc) / 4)
+        reinterpret_cast<uint32_t*>(a.job_out)[threadIdx.x] =
+            reinterpret_cast<const uint32_t*>(&a.job)[threadIdx.x];
     const T* __restrict__ uu = static_cast<const T*>(jd.uu);
     const T* __restrict__ vv = static_cast<const T*>(jd.vv);
     const T* __restrict__ ww = static_cast<const T*>(jd.ww);

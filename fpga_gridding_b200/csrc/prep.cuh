@@ -139,7 +139,11 @@ __device__ __forceinline__ int4 unpack_record(const uint2 r)
 // walks job j's points.
 struct PrepArgs
 {
+    // The jobs' table; where there is one job only and job_out is given, that
+    // job comes with the arguments and prep writes the table.
     const JobDesc* jobs;
+    JobDesc job;
+    JobDesc* job_out;
     int num_jobs;
     int blocks_per_job;
     int max_planes;          // row stride of plane_counts

@@ -350,8 +350,6 @@ cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
     if (n == 0) return cudaSuccess;
     const size_t tiles = sort_tiles(n);
     const SortTemp t = sort_temp(temp, n);
-    cudaError_t e = cudaMemsetAsync(temp, 0, radix_sort_temp_bytes(n), st);
-    if (e != cudaSuccess) return e;
     const unsigned cap = (unsigned)num_sms * 4u;
     const size_t want = (n + 8 * kHistThreads - 1) / (8 * kHistThreads);
     const unsigned blocks = want < cap ? (unsigned)want : cap;

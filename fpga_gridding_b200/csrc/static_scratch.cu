@@ -206,6 +206,7 @@ extern "C" int oskar_b200_grid_f_static(
     // The array keeps the last call's contents: clear what accumulates.
     B200_S(cudaMemsetAsync(counters, 0, 8 * (CNT_COUNT + 2), s));
     if (n) B200_S(cudaMemsetAsync(task_state, 0, 8 * task_tiles(n), s));
+    if (n) B200_S(cudaMemsetAsync(sort_tmp, 0, radix_sort_temp_bytes(n), s));
     B200_S(cudaMemsetAsync(plane_counts, 0, 8 * (size_t)P, s));
     st = static_cube_fill(conv_func, P, oversample, conv_size_half, d_planes,
                           slabs, d_norm_table, s);

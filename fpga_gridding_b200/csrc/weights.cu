@@ -398,7 +398,10 @@ int run_weights_write(oskar_B200Workspace* ws, int data_is_double,
                       unsigned long long* d_num_skipped, double frequency_hz,
                       cudaStream_t st)
 {
-    B200_TRY(ws->counters.ensure(sizeof(unsigned long long) * CNT_COUNT));
+    // The counters and, behind them, the sort's scratch start from zero.
+    const size_t zero_bytes = sizeof(unsigned long long) * CNT_COUNT +
+                              (ordered && n ? radix_sort_temp_bytes(n) : 0);
+    B200_TRY(ws->counters.ensure(zero_bytes));
     unsigned long long* skipped = skip_counter(ws, d_num_skipped);
     B200_TRY(cudaMemsetAsync(skipped, 0, sizeof(unsigned long long), st));
     int launches = 0;
@@ -428,11 +431,9 @@ int run_weights_write(oskar_B200Workspace* ws, int data_is_double,
     B200_TRY(ws->keys[1].ensure(4 * n));
     B200_TRY(ws->vals[0].ensure(4 * n));
     B200_TRY(ws->vals[1].ensure(4 * n));
-    B200_TRY(ws->sort_tmp.ensure(radix_sort_temp_bytes(n)));
     unsigned long long* counters =
         static_cast<unsigned long long*>(ws->counters.ptr);
-    B200_TRY(cudaMemsetAsync(counters, 0,
-                             sizeof(unsigned long long) * CNT_COUNT, st));
+    B200_TRY(cudaMemsetAsync(counters, 0, zero_bytes, st));
     unsigned long long* status = counters + CNT_STATUS;
     uint32_t* keys[2] = {static_cast<uint32_t*>(ws->keys[0].ptr),
                          static_cast<uint32_t*>(ws->keys[1].ptr)};
@@ -453,7 +454,7 @@ int run_weights_write(oskar_B200Workspace* ws, int data_is_double,
     ++launches;
     int which = 0;
     B200_TRY(radix_sort_pairs(keys, vals, n, bit_length(cells),
-                              ws->sort_tmp.ptr, status, ws->num_sms, st,
+                              counters + CNT_COUNT, status, ws->num_sms, st,
                               &which, &launches,
                               data_is_double
                                   ? nullptr
