@@ -360,7 +360,7 @@ def run_b200(args, world, rank, local):
     # Roofline of the dominant kernel (the Romein gridding kernel).
     kernel_ms = statistics.mean(grid_ms)
     cube_slab_bytes = cube.bytes
-    alg_bytes = n * (16 + 8) + 2 * g * g * 8 + cube_slab_bytes
+    alg_bytes = n * (8 + 4 + 8) + 2 * g * g * 8 + cube_slab_bytes
     achieved = alg_bytes / (kernel_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peaks()
     traffic = profiled_traffic()
@@ -1235,9 +1235,9 @@ def run_degrid(args, world, rank, local):
     ms = max_over_ranks(e0.elapsed_time(e1) / args.steps, world)
     taps = st.grid_updates
     kernel_ms = statistics.mean(kern_ms)
-    # per visibility: 16-byte record, 4-byte order value, 4-byte key, 8-byte
+    # per visibility: 8-byte record, 4-byte order value, 4-byte key, 8-byte
     # result; plus the grid read once and the kernel slabs
-    alg = n * (16 + 4 + 4 + 8) + g * g * 8 + cube.bytes
+    alg = n * (8 + 4 + 4 + 8) + g * g * 8 + cube.bytes
     peak, peak_kind = measured_peaks()
     achieved = alg / (kernel_ms * 1e-3) / 1e9
     out = {"metric": "degridding throughput (visibilities predicted)",

@@ -459,10 +459,9 @@ make_flush(const JobDesc& jd, int comp_part, bool active)
         return PlainFlush<GT>{static_cast<GT*>(jd.grid)};
 }
 
-// At least grid_ctas_per_sm<GT>() CTAs per SM.  FP32: with the
-// straight-line row slots and at most 6 rows per thread, 4 CTAs (64
-// registers) measured 16.28 ms at plain_large against 16.76 ms for 3 (and
-// 16.94-17.74 ms for 5 or 6 CTAs with at most 4 or 3 rows per thread).
+// At least grid_ctas_per_sm<GT>() CTAs per SM, with at most 6 rows per thread.
+// 39.2 M FP32 points: 4 CTAs (64 registers) 15.6 ms, 3 16.6, 5 16.2.  1.9 M
+// FP64 points: 3 CTAs (80 registers) 1692 us, 2 1860, 4 2406 (spills).
 template <typename GT, typename KT, bool STAGED, bool COMP, bool COUNT>
 __global__ void __launch_bounds__(kGridThreads, grid_ctas_per_sm<GT>())
 romein_grid_kernel(const GridArgs a)

@@ -1,7 +1,8 @@
 // Gridding of a batch of jobs on device-resident data:
 //   prep (placement, keys, norms, skip counts, plane histograms)
 //   -> one radix sort of (key, index) over all jobs (job in the top bits)
-//   -> task list (tasks never cross a job, tile or plane)
+//   -> task list (tasks never cross a job, tile or group of planes of one
+//      support)
 //   -> one persistent Romein gridding launch over every task of every job;
 //      each task gathers its points' records and visibilities through the
 //      sorted index (no separate permutation pass).
@@ -132,7 +133,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     if (time_slices < 1 || time_slices > kMaxBands ||
         (time_slices > 1 && (bands || degrid)))
         return OSKAR_B200_ERR_INVALID_ARGUMENT;
-    // (the error grid is folded in after the last band: not band-ordered)
+    // (the FP64 sums are folded in after the last band: not band-ordered)
     if (bands && (num_jobs != 1 || degrid || !bands->events ||
                   opt->accum_mode == OSKAR_B200_ACCUM_COMPENSATED))
         return OSKAR_B200_ERR_INVALID_ARGUMENT;

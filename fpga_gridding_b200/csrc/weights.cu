@@ -10,11 +10,11 @@
 // (one value per cell), row-major in v.
 //
 // write, ordered (the default, bit-exact): the reference adds the weights of
-//   a cell in point order, so a stable radix sort of (cell, point index)
-//   gathers each cell's points in that order, and they are added one after
-//   the other onto the cell's previous value (by one thread, or by one warp
-//   for a cell with more than 32 points).  The sums are the reference's to
-//   the bit for any weights.
+//   a cell in point order, so a stable radix sort of (cell, weight), or of
+//   (cell, point index) in FP64, gathers each cell's points in that order, and
+//   they are added one after the other onto the cell's previous value (by one
+//   thread, or by one warp for a cell with many points).  The sums are the
+//   reference's to the bit for any weights.
 // write, atomic: one fire-and-forget reduction per point.  Cell sums then
 //   depend on the order the reductions land in; they are exact whenever the
 //   partial sums are (e.g. unit weights below 2^24 per cell in FP32).
@@ -159,8 +159,8 @@ weights_key_kernel(size_t n, const T* __restrict__ uu,
 //
 // 39.2 M FP32 points, densest cells near 10^5 points: 307 us, against 2357
 // with point indices as values, 32 weights gathered one step ahead and the
-// windows dealt out in order; what must be moved takes 72 us, the rest is the
-// longest chain.
+// windows dealt out in order; reading keys and weights once takes 48 us, the
+// rest is the longest chain.
 constexpr int kSpan = 256;
 constexpr int kSumThreads = 256;
 constexpr int kSumCtasPerSm = 4;
