@@ -1,5 +1,5 @@
 // Gridding of a batch of jobs on device-resident data:
-//   prep (placement, keys, norms, skip counts, plane histograms)
+//   prep (placement, keys, norms, skip counts, grid updates)
 //   -> one radix sort of (key, index) over all jobs (job in the top bits)
 //   -> task list (tasks never cross a job, tile or group of planes of one
 //      support)
@@ -299,12 +299,10 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     }
     const int bpj = prep_blocks_per_job(max_points, num_jobs, ws->num_sms);
     // What starts from zero, in one buffer and one memset: the counters, then
-    // per job the skip count, the plane histogram and the ticket of its prep
-    // blocks (a word each, of which half is used), then the task list's tile
-    // words and the sort's scratch.
-    const size_t zero_words = CNT_COUNT +
-                              (size_t)num_jobs * (2 + (size_t)max_planes) +
-                              task_tiles(n);
+    // per job the skip count and the ticket of its prep blocks (a word each, of
+    // which half is used), then the task list's tile words and the sort's
+    // scratch.
+    const size_t zero_words = CNT_COUNT + 2 * (size_t)num_jobs + task_tiles(n);
     const size_t zero_bytes = sizeof(unsigned long long) * zero_words +
                               (n ? radix_sort_temp_bytes(n) : 0);
     B200_TRY(ws->counters.ensure(zero_bytes));
@@ -313,9 +311,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     unsigned long long* counters =
         static_cast<unsigned long long*>(ws->counters.ptr);
     unsigned long long* job_skipped = counters + CNT_COUNT;
-    unsigned long long* plane_counts = job_skipped + num_jobs;
-    unsigned long long* job_tickets =
-        plane_counts + (size_t)num_jobs * max_planes;
+    unsigned long long* job_tickets = job_skipped + num_jobs;
     unsigned long long* task_state = job_tickets + num_jobs;
     void* sort_temp = counters + zero_words;
     B200_TRY(cudaMemsetAsync(counters, 0, zero_bytes, st));
@@ -356,7 +352,6 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     pa.jobs = d_jobs;
     pa.num_jobs = num_jobs;
     pa.blocks_per_job = bpj;
-    pa.max_planes = max_planes;
     // (the norm is not a degridding output)
     pa.apply_weight = degrid ? 0 : opt->apply_weight;
     pa.key = kl;
@@ -369,7 +364,6 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     pa.counters = counters;
     pa.job_skipped = job_skipped;
     pa.norm_partials = static_cast<double*>(ws->partials.ptr);
-    pa.plane_counts = plane_counts;
     pa.job_tickets = reinterpret_cast<uint32_t*>(job_tickets);
 
     B200_TRY(mark(0));

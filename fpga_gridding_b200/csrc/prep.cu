@@ -1,7 +1,7 @@
 // Per-visibility preparation of a batch of jobs: placement (grid cell,
 // w-plane, oversample offsets, conjugation, skip test) exactly as
 // oskar_grid_wproj.c:70-101 computes it, the sort key, the skip counts, the
-// norms and the plane histograms; then, after the sort, the gridding work
+// norms and the grid updates; then, after the sort, the gridding work
 // list (tasks).
 #include <algorithm>
 #include <vector>
@@ -90,7 +90,6 @@ int prep_blocks_per_job(size_t max_points, int num_jobs, int num_sms)
 namespace {
 
 constexpr int kPrepThreads = 256;
-constexpr int kMaxSmemPlanes = 4096;
 
 // Spreads the low 16 bits of x to the even bit positions.
 __device__ __forceinline__ uint32_t spread_bits(uint32_t x)
@@ -135,6 +134,12 @@ __device__ __forceinline__ PlaceConsts place_consts(const JobDesc& jd)
     return pc;
 }
 
+// One point per thread and step.  The grid updates are summed per thread from
+// the supports; a histogram of planes by __match_any_sync and 16 KB of shared
+// counters, summed at the end, cost a tenth: 39.2 M FP32 points 441 -> 395 us,
+// 15.7 M 187 -> 168.  Bounded to 5, 6, 8 blocks per SM (48, 40, 32 registers):
+// 474, 467, 438 us against 395 unbounded (60 registers).  What must be moved
+// takes 144 us; the FP64 placement has the rest.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kPrepThreads)
 prep_kernel(const __grid_constant__ PrepArgs a)
@@ -151,23 +156,22 @@ prep_kernel(const __grid_constant__ PrepArgs a)
     const T* __restrict__ ww = static_cast<const T*>(jd.ww);
     const T* __restrict__ wt = static_cast<const T*>(jd.weight);
     const PlaceConsts pc = place_consts(jd);
-    const int num_planes = jd.num_planes, half = jd.half;
+    const PlaneDesc* __restrict__ planes = jd.planes;
+    const double* __restrict__ norm_table = jd.norm_table;
+    const int* __restrict__ support = jd.support;
+    const CoordScale scale = coord_scale(jd);
+    const int half = jd.half;
     const unsigned long long first = jd.first, n = jd.n;
-    __shared__ unsigned s_hist[kMaxSmemPlanes];
     __shared__ double s_norm[kPrepThreads / 32];
     __shared__ unsigned s_skip[kPrepThreads / 32];
-    const bool smem_hist = num_planes <= kMaxSmemPlanes;
-    if (smem_hist)
-        for (int p = threadIdx.x; p < num_planes; p += blockDim.x)
-            s_hist[p] = 0;
-    __syncthreads();
+    __shared__ unsigned long long s_updates[kPrepThreads / 32];
 
     const int span = 2 * half + 1;
     const uint32_t skip_key = 1u << a.key.total_bits;
     const int lane = threadIdx.x & 31;
-    unsigned long long* job_hist = a.plane_counts + (size_t)job * a.max_planes;
     double norm = 0.0;
     unsigned skipped = 0;
+    unsigned long long updates = 0;   // taps of the kept points
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t base = (size_t)blockIdx.x * blockDim.x; base < n;
          base += stride)
@@ -177,9 +181,9 @@ prep_kernel(const __grid_constant__ PrepArgs a)
         const size_t g = first + i;
         Placed p{};
         if (in_range)
-            p = place_one<T, MODE>(scale_coord(uu[i], jd),
-                                   scale_coord(vv[i], jd),
-                                   scale_coord(ww[i], jd), pc, jd.support);
+            p = place_one<T, MODE>(scale_coord(uu[i], scale),
+                                   scale_coord(vv[i], scale),
+                                   scale_coord(ww[i], scale), pc, support);
         const bool keep = in_range && !p.skipped;
         if (in_range)
         {
@@ -188,12 +192,14 @@ prep_kernel(const __grid_constant__ PrepArgs a)
                 a.rec[g] = pack_record(p, half);
                 a.keys[g] = make_key(a.key, job, p.gu, p.gv,
                                      a.key.by_plane
-                                         ? p.plane : jd.planes[p.plane].group);
-                double s = jd.norm_table[((size_t)p.plane * span +
+                                         ? p.plane : planes[p.plane].group);
+                double s = norm_table[((size_t)p.plane * span +
                                           (p.off_v + half)) * span +
                                          (p.off_u + half)];
                 if (a.apply_weight) s *= (double)wt[i];
                 norm += s;
+                const unsigned w = 2u * (unsigned)p.support + 1u;
+                updates += w * w;
             }
             else
             {
@@ -201,32 +207,28 @@ prep_kernel(const __grid_constant__ PrepArgs a)
             }
         }
         skipped += in_range && !keep;
-        // plane histogram, aggregated across equal planes in the warp
-        const unsigned pl = keep ? (unsigned)p.plane : 0xffffffffu;
-        const unsigned peers = __match_any_sync(0xffffffffu, pl);
-        if (keep && lane == __ffs(peers) - 1)
-        {
-            if (smem_hist) atomicAdd(&s_hist[pl], (unsigned)__popc(peers));
-            else atomicAdd(&job_hist[pl], (unsigned long long)__popc(peers));
-        }
     }
     norm = warp_sum(norm);
     skipped = warp_sum(skipped);
+    updates = warp_sum(updates);
     if (lane == 0)
     {
         s_norm[threadIdx.x >> 5] = norm;
         s_skip[threadIdx.x >> 5] = skipped;
+        s_updates[threadIdx.x >> 5] = updates;
     }
     __syncthreads();
     if (threadIdx.x == 0)
     {
         double t = 0.0;
-        unsigned long long k = 0;
+        unsigned long long k = 0, u = 0;
         for (int w = 0; w < kPrepThreads / 32; ++w)
         {
             t += s_norm[w];
             k += s_skip[w];
+            u += s_updates[w];
         }
+        if (u) atomicAdd(&a.counters[CNT_UPDATES], u);
         a.norm_partials[(size_t)job * gridDim.x + blockIdx.x] = t;
         if (k)
         {
@@ -234,14 +236,9 @@ prep_kernel(const __grid_constant__ PrepArgs a)
             atomicAdd(&a.counters[CNT_SKIPPED], k);
         }
     }
-    if (smem_hist)
-        for (int p = threadIdx.x; p < num_planes; p += blockDim.x)
-            if (s_hist[p])
-                atomicAdd(&job_hist[p], (unsigned long long)s_hist[p]);
     // The job's last block sums its norm partials in a fixed order
-    // (deterministic), adds them to the caller's norm, publishes the skip
-    // count, and counts grid updates from the plane histogram.  (As a kernel
-    // of its own this took a launch and 4 us.)
+    // (deterministic), adds them to the caller's norm and publishes the skip
+    // count.  (As a kernel of its own this took a launch and 4 us.)
     __shared__ bool s_last;
     __threadfence();
     __syncthreads();
@@ -250,36 +247,18 @@ prep_kernel(const __grid_constant__ PrepArgs a)
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    __shared__ unsigned long long s_updates[kPrepThreads / 32];
     norm = 0.0;
     for (unsigned k = threadIdx.x; k < gridDim.x; k += kPrepThreads)
         norm += __ldcg(&a.norm_partials[(size_t)job * gridDim.x + k]);
-    unsigned long long updates = 0;
-    for (int p = threadIdx.x; p < num_planes; p += kPrepThreads)
-    {
-        const unsigned long long w = 2ull * jd.support[p] + 1ull;
-        updates += __ldcg(&job_hist[p]) * w * w;
-    }
     norm = warp_sum(norm);
-    updates = warp_sum(updates);
-    if (lane == 0)
-    {
-        s_norm[threadIdx.x >> 5] = norm;
-        s_updates[threadIdx.x >> 5] = updates;
-    }
+    if (lane == 0) s_norm[threadIdx.x >> 5] = norm;
     __syncthreads();
     if (threadIdx.x == 0)
     {
         double t = 0.0;
-        unsigned long long u = 0;
-        for (int w = 0; w < kPrepThreads / 32; ++w)
-        {
-            t += s_norm[w];
-            u += s_updates[w];
-        }
+        for (int w = 0; w < kPrepThreads / 32; ++w) t += s_norm[w];
         if (jd.d_norm) *jd.d_norm += t;
         if (jd.d_skipped) *jd.d_skipped = __ldcg(&a.job_skipped[job]);
-        atomicAdd(&a.counters[CNT_UPDATES], u);
     }
 }
 

@@ -30,6 +30,7 @@ struct Placed
     int off_u, off_v;
     int conj;                   // -1 when w > 0, else +1
     int skipped;
+    int support;                // of the plane
 };
 
 __device__ __forceinline__ int sat_i32(long long x)
@@ -92,6 +93,7 @@ __device__ __forceinline__ Placed place_one(T u, T v, T w,
                                         (float)c.oversample));
     }
     const int s = support[p.plane];
+    p.support = s;
     p.skipped = (gu + s >= c.grid_size) || (gu - s < 0) ||
                 (gv + s >= c.grid_size) || (gv - s < 0);
     p.gu = (int)gu;
@@ -105,13 +107,22 @@ __device__ __forceinline__ Placed place_one(T u, T v, T w,
 // host: one multiplication in the data's precision (the FP64 scale rounded
 // to float for FP32 data).  The scale is exactly 1 when no frequency is
 // given, and x * 1 == x.
-__device__ __forceinline__ double scale_coord(double x, const JobDesc& jd)
+struct CoordScale
 {
-    return __dmul_rn(x, jd.coord_scale);
+    double d;
+    float f;
+};
+__device__ __forceinline__ CoordScale coord_scale(const JobDesc& jd)
+{
+    return CoordScale{jd.coord_scale, jd.coord_scale_f};
 }
-__device__ __forceinline__ float scale_coord(float x, const JobDesc& jd)
+__device__ __forceinline__ double scale_coord(double x, const CoordScale& c)
 {
-    return __fmul_rn(x, jd.coord_scale_f);
+    return __dmul_rn(x, c.d);
+}
+__device__ __forceinline__ float scale_coord(float x, const CoordScale& c)
+{
+    return __fmul_rn(x, c.f);
 }
 
 // Placement record of a kept point, 8 bytes: x = gu | gv << 16 (grids are at
@@ -146,7 +157,6 @@ struct PrepArgs
     JobDesc* job_out;
     int num_jobs;
     int blocks_per_job;
-    int max_planes;          // row stride of plane_counts
     int apply_weight;
     KeyLayout key;
     uint2* rec;              // [total points], global index
@@ -154,7 +164,6 @@ struct PrepArgs
     unsigned long long* counters;     // CNT_SKIPPED: all jobs
     unsigned long long* job_skipped;  // [num_jobs]
     double* norm_partials;            // [num_jobs][blocks_per_job]
-    unsigned long long* plane_counts; // [num_jobs][max_planes]
     uint32_t* job_tickets;            // [num_jobs]: blocks that are done
 };
 

@@ -147,7 +147,6 @@ extern "C" int oskar_b200_grid_f_static(
     auto* d_planes = cv.take<PlaneDesc>(sizeof(PlaneDesc) * P);
     auto* d_support = cv.take<int>(sizeof(int) * P);
     auto* d_norm_table = cv.take<double>(sizeof(double) * P * span * span);
-    auto* plane_counts = cv.take<unsigned long long>(8 * (size_t)P);
     auto* partials = cv.take<double>(8 * (size_t)bpj);
     auto* slabs = cv.take<float2>(slab_bytes);
     uint32_t* keys[2] = {cv.take<uint32_t>(4 * n), cv.take<uint32_t>(4 * n)};
@@ -207,7 +206,6 @@ extern "C" int oskar_b200_grid_f_static(
     B200_S(cudaMemsetAsync(counters, 0, 8 * (CNT_COUNT + 2), s));
     if (n) B200_S(cudaMemsetAsync(task_state, 0, 8 * task_tiles(n), s));
     if (n) B200_S(cudaMemsetAsync(sort_tmp, 0, radix_sort_temp_bytes(n), s));
-    B200_S(cudaMemsetAsync(plane_counts, 0, 8 * (size_t)P, s));
     st = static_cube_fill(conv_func, P, oversample, conv_size_half, d_planes,
                           slabs, d_norm_table, s);
     if (st) return st;
@@ -216,7 +214,6 @@ extern "C" int oskar_b200_grid_f_static(
     pa.jobs = d_job;
     pa.num_jobs = 1;
     pa.blocks_per_job = bpj;
-    pa.max_planes = P;
     pa.apply_weight = 0;
     pa.key = kl;
     pa.rec = rec;
@@ -224,7 +221,6 @@ extern "C" int oskar_b200_grid_f_static(
     pa.counters = counters;
     pa.job_skipped = job_skipped;
     pa.norm_partials = partials;
-    pa.plane_counts = plane_counts;
     pa.job_tickets = job_ticket;
     B200_S(launch_prep(pa, 0, OSKAR_B200_COORDS_F64, s));
     if (n == 0) return OSKAR_B200_OK;
