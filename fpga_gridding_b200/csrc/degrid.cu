@@ -515,15 +515,24 @@ cudaError_t launch_variant(const uint32_t* order, const uint32_t* sorted_keys,
 cudaError_t launch_degrid(const uint32_t* order, const uint32_t* sorted_keys,
                           const uint2* rec, const JobDesc* jobs, int job_shift,
                           int apply_weight, unsigned long long* counters,
-                          size_t n,
+                          size_t n, int max_support,
                           int data_is_double, int kernel_type, int num_sms,
                           cudaStream_t st)
 {
     // Chunks of 256 share most; fewer than the 4 resident CTAs per SM leave
     // SMs idle, so small calls take 128, 64 or 32: 23 thousand FP64 points,
-    // supports 5 to 30, 450 -> 213 us a call.
+    // supports 5 to 30, 450 -> 213 us a call.  Below 8 chunks of 256 per
+    // resident CTA, the last chunks of a wide support are waited for, so there
+    // a chunk's taps are bounded too: 531 thousand points, supports 4 to 34,
+    // 583 us with 256, 485 with 128, 448 with 32; at narrow supports (242
+    // thousand points, 4 to 16) 64 instead of 256 cost 129 -> 149 us.
+    const int w = 2 * max_support + 1;
+    const size_t resident = (size_t)num_sms * 4;
     int chunk = kDegridChunk;
-    while (chunk > 32 && n < (size_t)num_sms * 4 * chunk) chunk /= 2;
+    while (chunk > 32 &&
+           (n < resident * chunk ||
+            (n < resident * 8 * kDegridChunk && chunk * w * w > 300000)))
+        chunk /= 2;
     // up to 8 CTAs of 8 warps per SM, persistent over the work queue
     const size_t want = (n + chunk - 1) / chunk;
     const size_t cap = (size_t)num_sms * 8;

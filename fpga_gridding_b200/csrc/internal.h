@@ -312,8 +312,8 @@ cudaError_t launch_slice_bounds(const unsigned long long* counters,
 cudaError_t launch_degrid(const uint32_t* order, const uint32_t* sorted_keys,
                           const uint2* rec, const JobDesc* jobs, int job_shift,
                           int apply_weight, unsigned long long* counters,
-                          size_t n, int data_is_double, int kernel_type,
-                          int num_sms, cudaStream_t st);
+                          size_t n, int max_support, int data_is_double,
+                          int kernel_type, int num_sms, cudaStream_t st);
 
 int run_grid(oskar_B200Workspace* ws, const oskar_B200Cube* cube,
              const oskar_B200Options* opt, size_t num_points, const void* uu,

@@ -152,6 +152,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     // Job table (host, pinned: it is the source of an async upload).
     size_t n = 0, max_points = 0, comp_cells = 0;
     int max_grid = 1, max_planes = 1, max_groups = 1;
+    int max_support = 0;
     unsigned max_block = 0;
     for (int j = 0; j < num_jobs; ++j)
     {
@@ -161,6 +162,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         max_planes = std::max(max_planes, jobs[j].cube->num_planes);
         max_groups = std::max(max_groups,
                               (int)jobs[j].cube->group_support.size());
+        max_support = std::max(max_support, jobs[j].cube->max_support);
         max_block = std::max(max_block, jobs[j].cube->max_block_bytes);
         if (comp)
             comp_cells += (size_t)jobs[j].grid_size * jobs[j].grid_size;
@@ -395,7 +397,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         B200_TRY(mark(3));
         B200_TRY(launch_degrid(vals[which], keys[which], pa.rec, d_jobs,
                                kl.job_shift, opt->apply_weight, counters, n,
-                               dbl, c0->kernel_type, ws->num_sms, st));
+                               max_support, dbl, c0->kernel_type, ws->num_sms, st));
         launches += 1;
         B200_TRY(mark(4));
         ws->events_recorded = timing ? 1 : 0;
