@@ -57,6 +57,7 @@ EXPORTED_SYMBOLS = (
     "oskar_b200_server_free",
     "oskar_b200_selftest_bounded_wait",
     "oskar_b200_testing_fail_allocation",
+    "oskar_b200_testing_expire_wait",
     "oskar_b200_testing_set_static_status",
     "oskar_b200_build_info",
 )
@@ -223,6 +224,8 @@ def load():
     lib.oskar_b200_testing_set_static_status.restype = C.c_int
     lib.oskar_b200_testing_fail_allocation.argtypes = [C.c_longlong]
     lib.oskar_b200_testing_fail_allocation.restype = C.c_int
+    lib.oskar_b200_testing_expire_wait.argtypes = [_P, C.c_int, C.c_uint]
+    lib.oskar_b200_testing_expire_wait.restype = C.c_int
     lib.oskar_b200_selftest_bounded_wait.argtypes = [_P, C.c_uint,
                                                      C.POINTER(C.c_int)]
     lib.oskar_b200_selftest_bounded_wait.restype = C.c_int

@@ -1681,3 +1681,18 @@ int oskar_b200_degrid_host(oskar_B200Workspace* ws, const oskar_B200Cube* cube,
 }
 
 }  // extern "C"
+
+extern "C" int oskar_b200_testing_expire_wait(oskar_B200Workspace* ws,
+                                              int stage, unsigned tile)
+{
+    if (stage < 0 || stage > 2) return OSKAR_B200_ERR_INVALID_ARGUMENT;
+    if (!ws)
+    {
+        int st = dropin_workspace(&ws);
+        if (st) return st;
+    }
+    ws->expired = ExpiredWait{};
+    if (stage == 1) ws->expired.sort_tile = tile;
+    if (stage == 2) ws->expired.task_tile = tile;
+    return OSKAR_B200_OK;
+}

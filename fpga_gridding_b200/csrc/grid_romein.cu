@@ -497,7 +497,7 @@ romein_grid_kernel(const GridArgs a)
     __shared__ int s_warp_heads[kGridThreads / 32];
 
     unsigned long long* status = &a.counters[CNT_STATUS];
-    const unsigned num_tasks = (unsigned)a.counters[CNT_TASKS];
+    const unsigned num_tasks = tasks_listed(a.counters);
     unsigned long long first = 0, end = num_tasks;
     unsigned long long* queue = &a.counters[CNT_TASK_NEXT];
     if (a.range)

@@ -116,6 +116,15 @@ struct BandPlan
     int order[kMaxBands];     // set by run_batch
 };
 
+// A tile whose look-back counts as expired (testing aid): of the sort, of the
+// task list, or of neither.
+constexpr unsigned kNoTile = 0xffffffffu;
+struct ExpiredWait
+{
+    unsigned sort_tile = kNoTile;
+    unsigned task_tile = kNoTile;
+};
+
 }  // namespace b200
 
 // Opaque public types.
@@ -176,6 +185,9 @@ struct oskar_B200Workspace
     int tuned_tile_shift = 0;
     int tuned_staging = 2;
     int tuned_comp_radius = 0;
+    // bounded wait that later calls treat as expired
+    // (oskar_b200_testing_expire_wait)
+    b200::ExpiredWait expired;
 };
 
 struct oskar_B200Cube
@@ -218,12 +230,14 @@ size_t radix_sort_temp_bytes(size_t n);
 // 0 .. n - 1 where that is null.  The sorted pairs end in
 // keys[*which] / vals[*which].  *status: the device status word; when it has
 // DEV_ERR_TIMEOUT (set here when a bounded wait expires) the pairs are not to
-// be used.  temp: radix_sort_temp_bytes(n) zeroed bytes.
+// be used.  temp: radix_sort_temp_bytes(n) zeroed bytes.  expired_tile: the
+// tile whose look-back counts as expired, for tests.
 cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
                              int num_bits, void* temp,
                              unsigned long long* status, int num_sms,
                              cudaStream_t st, int* which, int* launches,
-                             const uint32_t* first_vals = nullptr);
+                             const uint32_t* first_vals = nullptr,
+                             unsigned expired_tile = kNoTile);
 
 // ---- cube.cu ----------------------------------------------------------------
 // d_conv_im == nullptr: d_conv_func is the interleaved complex cube;

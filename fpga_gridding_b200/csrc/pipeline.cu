@@ -390,7 +390,8 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     int which = 0;
     B200_TRY(radix_sort_pairs(keys, vals, n, kl.total_bits + 1,
                               sort_temp, counters + CNT_STATUS,
-                              ws->num_sms, st, &which, &launches));
+                              ws->num_sms, st, &which, &launches, nullptr,
+                              ws->expired.sort_tile));
     B200_TRY(mark(2));
     if (degrid)
     {
@@ -414,7 +415,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
                           task_state,
                           static_cast<uint32_t*>(ws->task_start.ptr),
                           static_cast<uint32_t*>(ws->task_job.ptr), st,
-                          &launches));
+                          &launches, ws->expired.task_tile));
 
     GridArgs ga{};
     ga.order = vals[which];
@@ -645,7 +646,7 @@ __global__ void slice_bounds_kernel(const unsigned long long* counters,
                                     int k_slices, uint32_t* first,
                                     unsigned long long* queues)
 {
-    const unsigned long long t = counters[CNT_TASKS];
+    const unsigned long long t = tasks_listed(counters);
     for (int k = threadIdx.x; k <= k_slices; k += blockDim.x)
     {
         first[k] = (uint32_t)(t * (unsigned long long)k /

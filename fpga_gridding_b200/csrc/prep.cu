@@ -308,7 +308,8 @@ __global__ void __launch_bounds__(kTaskThreads)
 task_list_kernel(const uint32_t* __restrict__ keys, size_t n,
                  unsigned long long* __restrict__ counters, int fine_key_bits,
                  const TaskSizes sizes, int job_shift,
-                 unsigned long long* state, uint32_t* __restrict__ task_start,
+                 unsigned long long* state, unsigned expired_tile,
+                 uint32_t* __restrict__ task_start,
                  uint32_t* __restrict__ task_job)
 {
     __shared__ unsigned s_tile, s_base;
@@ -371,7 +372,8 @@ task_list_kernel(const uint32_t* __restrict__ keys, size_t n,
         volatile unsigned long long* word = state + tile;
         if (lane == 0) *word = (tile ? 1ull : 2ull) << 62 | total;
         unsigned before = 0;
-        const bool ok = tasks_before(state, tile, &before);
+        const bool ok = tile != expired_tile &&
+                        tasks_before(state, tile, &before);
         if (lane == 0)
         {
             if (ok)
@@ -453,14 +455,15 @@ cudaError_t launch_tasks(const uint32_t* sorted_keys, size_t n,
                          unsigned long long* counters, int fine_key_bits,
                          int job_shift, const TaskSizes& sizes,
                          unsigned long long* tile_state, uint32_t* task_start,
-                         uint32_t* task_job, cudaStream_t st, int* launches)
+                         uint32_t* task_job, cudaStream_t st, int* launches,
+                         unsigned expired_tile)
 {
     const size_t tiles = task_tiles(n);
     if (tiles == 0) return cudaSuccess;
     if (launches) *launches += 1;
     task_list_kernel<<<(unsigned)tiles, kTaskThreads, 0, st>>>(
         sorted_keys, n, counters, fine_key_bits, sizes, job_shift, tile_state,
-        task_start, task_job);
+        expired_tile, task_start, task_job);
     return cudaGetLastError();
 }
 
@@ -482,7 +485,7 @@ __global__ void band_first_kernel(const uint32_t* __restrict__ sorted_keys,
                                   int band_shift, uint32_t band_mask,
                                   int num_bands, uint32_t* __restrict__ band_first)
 {
-    const unsigned nt = (unsigned)counters[CNT_TASKS];
+    const unsigned nt = tasks_listed(counters);
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t <= nt;
          t += (size_t)gridDim.x * blockDim.x)
     {

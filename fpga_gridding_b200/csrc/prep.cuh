@@ -176,13 +176,25 @@ cudaError_t launch_prep(const PrepArgs& a, int data_is_double, int coord_mode,
                         cudaStream_t st);
 // Task list: a task starts where (job, coarse tile, group) changes and every
 // 2^log2_max positions; task_job[t] is the job of task t.  tile_state: a zeroed
-// word per tile (task_tiles(n)); counters[CNT_TASK_TILE] is zero.
+// word per tile (task_tiles(n)); counters[CNT_TASK_TILE] is zero.  A tile whose
+// wait for the tiles before it expires sets DEV_ERR_TIMEOUT and leaves a hole in
+// the list, whatever CNT_TASKS says: the kernels that read the list look at the
+// status word first (tasks_listed).  expired_tile: as in radix_sort_pairs.
 size_t task_tiles(size_t n);
 cudaError_t launch_tasks(const uint32_t* sorted_keys, size_t n,
                          unsigned long long* counters, int fine_key_bits,
                          int job_shift, const TaskSizes& sizes,
                          unsigned long long* tile_state, uint32_t* task_start,
-                         uint32_t* task_job, cudaStream_t st, int* launches);
+                         uint32_t* task_job, cudaStream_t st, int* launches,
+                         unsigned expired_tile = kNoTile);
+// The tasks that the kernels behind the task list may take: none when the sort
+// or the list gave up (counters[CNT_TASKS] may count entries never written).
+__device__ __forceinline__ unsigned tasks_listed(
+    const unsigned long long* counters)
+{
+    return counters[CNT_STATUS] & DEV_ERR_TIMEOUT
+               ? 0u : (unsigned)counters[CNT_TASKS];
+}
 // Bands of a single job's task list: band b holds the tasks of coarse-tile
 // row b; band_first[b] (b <= num_bands) is its first task.
 cudaError_t launch_band_first(const uint32_t* sorted_keys,

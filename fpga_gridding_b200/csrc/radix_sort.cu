@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(kSortThreads, 3)
 rs_pass_kernel(const uint32_t* __restrict__ keys_in,
                const uint32_t* __restrict__ vals_in, size_t n, int pass,
                uint32_t mask, SortTemp t, unsigned long long* status,
-               uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out)
+               unsigned expired_tile, uint32_t* __restrict__ keys_out,
+               uint32_t* __restrict__ vals_out)
 {
     __shared__ uint16_t s_count[kSortWarps][kRadix];
     // The tile's pairs in digit order; before that, the lanes of each warp
@@ -303,7 +304,8 @@ rs_pass_kernel(const uint32_t* __restrict__ keys_in,
     if (d < kRadix)
     {
         uint32_t before = 0;
-        ok = look_back(col, kRadix, tile, tag, &before);
+        ok = s_tile != expired_tile &&
+             look_back(col, kRadix, tile, tag, &before);
         if (ok && tile != 0)
             store_word(col + tile * kRadix,
                        kTilePrefix | tag_bits | (before + total));
@@ -344,7 +346,8 @@ cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
                              int num_bits, void* temp,
                              unsigned long long* status, int num_sms,
                              cudaStream_t st, int* which, int* launches,
-                             const uint32_t* first_vals)
+                             const uint32_t* first_vals,
+                             unsigned expired_tile)
 {
     *which = 0;
     if (n == 0) return cudaSuccess;
@@ -363,7 +366,7 @@ cudaError_t radix_sort_pairs(uint32_t* keys[2], uint32_t* vals[2], size_t n,
         const int bits = num_bits - 8 * pass < 8 ? num_bits - 8 * pass : 8;
         rs_pass_kernel<<<(unsigned)tiles, kSortThreads, 0, st>>>(
             keys[cur], pass ? vals[cur] : first_vals, n, pass, (1u << bits) - 1u,
-            t, status, keys[cur ^ 1], vals[cur ^ 1]);
+            t, status, expired_tile, keys[cur ^ 1], vals[cur ^ 1]);
         if (launches) *launches += 1;
         cur ^= 1;
     }

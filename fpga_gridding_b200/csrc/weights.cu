@@ -458,7 +458,8 @@ int run_weights_write(oskar_B200Workspace* ws, int data_is_double,
                               &which, &launches,
                               data_is_double
                                   ? nullptr
-                                  : static_cast<const uint32_t*>(weight)));
+                                  : static_cast<const uint32_t*>(weight),
+                              ws->expired.sort_tile));
     const size_t sum_want = (n + kSumThreads / 32 * kSpan - 1) /
                             (kSumThreads / 32 * kSpan);
     const int sum_blocks = (int)std::min<size_t>(

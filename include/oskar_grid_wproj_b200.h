@@ -638,6 +638,15 @@ OSKAR_B200_EXPORT int oskar_b200_selftest_bounded_wait(
  * without exhausting a shared GPU.  Process-wide; not for production use. */
 OSKAR_B200_EXPORT int oskar_b200_testing_fail_allocation(long long after);
 
+/* Testing aid for the bounded waits between the blocks of one launch (no
+ * counterpart in the reference): later calls on this workspace behave as if
+ * the wait of tile `tile` (4096 positions each) had expired, in the sort
+ * (stage 1) or in the task list (stage 2); stage 0 disarms.  No block waits
+ * any longer for it.  ws NULL: the calling thread's workspace of the
+ * reference's own entry points. */
+OSKAR_B200_EXPORT int oskar_b200_testing_expire_wait(oskar_B200Workspace* ws,
+        int stage, unsigned tile);
+
 /* Testing aid for oskar_b200_grid_f_static_status (no counterpart in the
  * reference): enqueues on `stream` a write of `bits` (device check bits:
  * 1 grid index, 2 slab index, 4 wait timeout, 8 task bounds) into the
