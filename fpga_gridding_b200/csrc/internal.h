@@ -151,8 +151,10 @@ struct oskar_B200Workspace
     // drop-in staging of the caller's host arrays
     b200::DeviceBuffer in_uu, in_vv, in_ww, in_vis, in_weight, in_grid,
         in_cube, in_norm;
-    // FP64 sums of ACCUM_COMPENSATED
+    // FP64 sums of ACCUM_COMPENSATED, and the smallest size in bytes at which
+    // both planes of them did not fit (0: none yet)
     b200::DeviceBuffer comp_grid;
+    size_t comp_refused = 0;
     // drop-in pipelined upload: copy stream, its events (cube, one per
     // chunk) and the zeroed grid the chunks accumulate into
     cudaStream_t copy_stream = nullptr;

@@ -126,6 +126,31 @@ static TaskSizes task_sizes(const KeyLayout& kl, int num_jobs,
     return t;
 }
 
+// The FP64 sums of `cells` cells: *planes = 2 (real and imaginary parts), or 1
+// where there is no room for both; the tasks then run twice and share one plane.
+// A size that did not fit once is not tried again, nor is any above it: a try
+// frees the plane at hand first, which waits for the device and leaves captured
+// graphs with a pointer to freed memory.  Under capture nothing grows that one
+// plane suffices for.
+static cudaError_t compensated_sums(oskar_B200Workspace* ws, size_t cells,
+                                    bool capturing, int* planes)
+{
+    const size_t one = cells * sizeof(double), both = 2 * one;
+    DeviceBuffer& sums = ws->comp_grid;
+    *planes = 2;
+    if (sums.ptr && sums.bytes >= both) return cudaSuccess;
+    const bool refused = ws->comp_refused && both >= ws->comp_refused;
+    const bool has_one = sums.ptr && sums.bytes >= one;
+    if (!refused && !(capturing && has_one))
+    {
+        const cudaError_t e = sums.ensure(both);
+        if (e != cudaErrorMemoryAllocation) return e;
+        ws->comp_refused = both;
+    }
+    *planes = 1;
+    return sums.ensure(one);
+}
+
 int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
               int num_jobs, const HostJob* jobs, cudaStream_t st,
               bool degrid, BandPlan* bands, int time_slices)
@@ -246,14 +271,49 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
             B200_TRY(cudaEventSynchronize(ws->jobs_event[slot]));
         ws->jobs_event_pending[slot] = 0;
     }
-    // FP64 sums of the real and of the imaginary parts.  Where there is no
-    // room for both, the tasks run twice and share one plane of sums.
-    int comp_passes = comp ? 1 : 0;
-    if (comp && ws->comp_grid.ensure(2 * comp_cells * sizeof(double)) !=
-                    cudaSuccess)
+    const int bpj = prep_blocks_per_job(max_points, num_jobs, ws->num_sms);
+    // What starts from zero, in one buffer and one memset: the counters, then
+    // per job the skip count and the ticket of its prep blocks (a word each, of
+    // which half is used), then the task list's tile words and the sort's
+    // scratch.
+    const size_t zero_words = CNT_COUNT + 2 * (size_t)num_jobs + task_tiles(n);
+    const size_t zero_bytes = sizeof(unsigned long long) * zero_words +
+                              (n ? radix_sort_temp_bytes(n) : 0);
+    auto buffers = [&]() -> cudaError_t {
+        cudaError_t e = ws->counters.ensure(zero_bytes);
+        auto also = [&](DeviceBuffer& b, size_t bytes) {
+            if (e == cudaSuccess) e = b.ensure(bytes);
+        };
+        also(ws->jobs, job_bytes);
+        also(ws->partials, sizeof(double) * num_jobs * bpj);
+        if (n == 0) return e;
+        also(ws->keys[0], 4 * n);
+        also(ws->keys[1], 4 * n);
+        also(ws->vals[0], 4 * n);
+        also(ws->vals[1], 4 * n);
+        also(ws->rec, sizeof(uint2) * n);
+        if (degrid) return e;
+        also(ws->task_start, 4 * (n + 2));
+        also(ws->task_job, 4 * (n + 2));
+        return e;
+    };
+    cudaError_t be = buffers();
+    // The FP64 sums come last, so that the second plane takes only what the
+    // rest leaves; one that an earlier call left is given up for the rest.
+    if (be == cudaErrorMemoryAllocation && comp && !capturing &&
+        ws->comp_grid.bytes >= 2 * comp_cells * sizeof(double))
     {
-        comp_passes = 2;
-        B200_TRY(ws->comp_grid.ensure(comp_cells * sizeof(double)));
+        ws->comp_grid.release();
+        ws->comp_refused = 2 * comp_cells * sizeof(double);
+        be = buffers();
+    }
+    B200_TRY(be);
+    int comp_passes = 0;
+    if (comp)
+    {
+        int planes = 0;
+        B200_TRY(compensated_sums(ws, comp_cells, capturing, &planes));
+        comp_passes = 3 - planes;
     }
     PrepArgs pa{};
     JobDesc* hj = num_jobs == 1 ? &pa.job
@@ -299,17 +359,6 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         first += h.num_points;
         comp_off += (size_t)h.grid_size * h.grid_size;
     }
-    const int bpj = prep_blocks_per_job(max_points, num_jobs, ws->num_sms);
-    // What starts from zero, in one buffer and one memset: the counters, then
-    // per job the skip count and the ticket of its prep blocks (a word each, of
-    // which half is used), then the task list's tile words and the sort's
-    // scratch.
-    const size_t zero_words = CNT_COUNT + 2 * (size_t)num_jobs + task_tiles(n);
-    const size_t zero_bytes = sizeof(unsigned long long) * zero_words +
-                              (n ? radix_sort_temp_bytes(n) : 0);
-    B200_TRY(ws->counters.ensure(zero_bytes));
-    B200_TRY(ws->jobs.ensure(job_bytes));
-    B200_TRY(ws->partials.ensure(sizeof(double) * num_jobs * bpj));
     unsigned long long* counters =
         static_cast<unsigned long long*>(ws->counters.ptr);
     unsigned long long* job_skipped = counters + CNT_COUNT;
@@ -336,20 +385,6 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
         }
     }
     const JobDesc* d_jobs = static_cast<const JobDesc*>(ws->jobs.ptr);
-
-    if (n > 0)
-    {
-        B200_TRY(ws->keys[0].ensure(4 * n));
-        B200_TRY(ws->keys[1].ensure(4 * n));
-        B200_TRY(ws->vals[0].ensure(4 * n));
-        B200_TRY(ws->vals[1].ensure(4 * n));
-        B200_TRY(ws->rec.ensure(sizeof(uint2) * n));
-        if (!degrid)
-        {
-            B200_TRY(ws->task_start.ensure(4 * (n + 2)));
-            B200_TRY(ws->task_job.ensure(4 * (n + 2)));
-        }
-    }
 
     pa.jobs = d_jobs;
     pa.num_jobs = num_jobs;
