@@ -843,10 +843,11 @@ int oskar_b200_last_stats(oskar_B200Workspace* ws, oskar_B200Stats* stats)
     stats->grid_updates = c[CNT_UPDATES];
     stats->num_tasks = c[CNT_TASKS];
     stats->atomic_flushes = c[CNT_FLUSHES];
-    stats->status = c[CNT_STATUS] ? (c[CNT_STATUS] & DEV_ERR_TIMEOUT
-                                         ? OSKAR_B200_ERR_TIMEOUT
-                                         : OSKAR_B200_ERR_DEVICE_CHECK)
-                                  : OSKAR_B200_OK;
+    const unsigned long long bits = c[CNT_STATUS] | c[CNT_WEIGHTS_STATUS];
+    stats->status = bits ? (bits & DEV_ERR_TIMEOUT
+                                ? OSKAR_B200_ERR_TIMEOUT
+                                : OSKAR_B200_ERR_DEVICE_CHECK)
+                         : OSKAR_B200_OK;
     stats->kernel_launches = ws->last_launches;
     if (ws->events_recorded)
     {

@@ -222,6 +222,9 @@ enum CounterSlot
     CNT_STATUS = 4,      // DEV_ERR_* bits
     CNT_UPDATES = 5,     // grid updates (taps) of gridded points
     CNT_TASK_TILE = 6,   // ticket of the task list's tiles
+    // host mirror only (the device word stays zero): DEV_ERR_* bits of the
+    // ordered weights write since the last gridding or degridding call
+    CNT_WEIGHTS_STATUS = 7,
     CNT_COUNT = 8
 };
 
@@ -351,7 +354,7 @@ int measure_atomic_rate(oskar_B200Workspace* ws, void* grid, int grid_size,
 
 // ---- weights.cu -------------------------------------------------------------
 // Skip count left by an ordered write whose sort gave up (the grid is then
-// unchanged).
+// unchanged, and the status goes to h_counters[CNT_WEIGHTS_STATUS]).
 constexpr unsigned long long kSortFailed = ~0ull;
 // Uniform weighting (utils/oskar_grid_weights.c:38-172) on device arrays.
 // *d_num_skipped (or a workspace counter when null) is reset, then counts.

@@ -185,15 +185,20 @@ weights_run_sum_kernel(size_t n, const uint32_t* __restrict__ keys,
                        const T* __restrict__ weight, uint32_t sentinel,
                        T* __restrict__ grid,
                        const unsigned long long* __restrict__ status,
+                       unsigned long long* __restrict__ host_status,
                        unsigned long long* __restrict__ queue,
                        unsigned long long* __restrict__ skipped)
 {
     constexpr unsigned kAll = 0xffffffffu;
     // (four more: a lane reads its run four values at a time)
     __shared__ __align__(16) T s_v[kSumThreads / 32][kSpan + 4];
+    // The status goes to the host from here (pinned memory; a copy of its own
+    // would cost a launch).
+    const bool reports = blockIdx.x == 0 && threadIdx.x == 0;
+    if (reports) *host_status = *status;
     if (*status)   // the sort gave up: its pairs are not to be used
     {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *skipped = kSortFailed;
+        if (reports) *skipped = kSortFailed;
         return;
     }
     const int lane = threadIdx.x & 31;
@@ -462,16 +467,20 @@ int run_weights_write(oskar_B200Workspace* ws, int data_is_double,
                               ws->expired.sort_tile));
     const size_t sum_want = (n + kSumThreads / 32 * kSpan - 1) /
                             (kSumThreads / 32 * kSpan);
+    unsigned long long* host_status =
+        static_cast<unsigned long long*>(ws->h_counters) + CNT_WEIGHTS_STATUS;
     const int sum_blocks = (int)std::min<size_t>(
         sum_want, (size_t)ws->num_sms * kSumCtasPerSm);
     if (data_is_double)
         weights_run_sum_kernel<double><<<sum_blocks, kSumThreads, 0, st>>>(
             n, keys[which], vals[which], (const double*)weight, sentinel,
-            (double*)grid, status, counters + CNT_TASK_NEXT, skipped);
+            (double*)grid, status, host_status, counters + CNT_TASK_NEXT,
+            skipped);
     else
         weights_run_sum_kernel<float><<<sum_blocks, kSumThreads, 0, st>>>(
             n, keys[which], vals[which], (const float*)weight, sentinel,
-            (float*)grid, status, counters + CNT_TASK_NEXT, skipped);
+            (float*)grid, status, host_status, counters + CNT_TASK_NEXT,
+            skipped);
     B200_TRY(cudaGetLastError());
     ++launches;
     ws->last_launches = launches;

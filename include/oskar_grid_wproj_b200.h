@@ -389,7 +389,9 @@ OSKAR_B200_EXPORT int oskar_b200_place(oskar_B200Workspace* ws,
  *   oskar_grid_weights_write_{d,f} (stable sort by cell, then one
  *   sequential sum per cell); ordered = 0 issues one atomic add per point
  *   (faster; cell sums depend on the order the atomics land in, exact when
- *   every partial sum is, e.g. unit weights).
+ *   every partial sum is, e.g. unit weights).  An ordered write whose sort
+ *   gave up a bounded wait leaves the grid as it was, sets *d_num_skipped to
+ *   UINT64_MAX and shows OSKAR_B200_ERR_TIMEOUT in oskar_b200_last_stats.
  * read: weight_out[i] = weight_in[i] / grid[cell] (0 for an empty cell);
  *   skipped points keep their weight_out value. */
 OSKAR_B200_EXPORT int oskar_b200_weights_write(oskar_B200Workspace* ws,
@@ -426,8 +428,9 @@ OSKAR_B200_EXPORT int oskar_b200_blocks_finish(oskar_B200Blocks* blocks,
         unsigned long long* num_skipped);
 OSKAR_B200_EXPORT int oskar_b200_blocks_free(oskar_B200Blocks* blocks);
 
-/* Statistics of the most recent oskar_b200_grid call on this workspace
- * (valid once its stream has been synchronised). */
+/* Statistics of the most recent gridding or degridding call on this workspace
+ * (valid once its stream has been synchronised).  `status` covers that call
+ * and the last ordered weights write behind it, if there was one. */
 typedef struct oskar_B200Stats
 {
     unsigned long long num_points;     /* visibilities given */
