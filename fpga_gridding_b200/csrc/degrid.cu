@@ -31,6 +31,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "degrid_plan.h"
 #include "internal.h"
 #include "prep.cuh"
 #include "task_order.cuh"
@@ -47,7 +48,6 @@ constexpr int kGroup = 16;          // lanes per visibility
 constexpr int kGroups = 32 / kGroup;
 constexpr int kDegridMaxW = 255;   // footprint width for support <= 127
 constexpr int kPairMaxW = 48;      // widest footprint gathered in pairs
-constexpr int kDegridChunk = 256;  // visibilities per work-queue item, at most
 
 // Sum over taps of grid * conj(Kt), Kt = (kr, sgn * ki).  FP32: two packed
 // FMAs per tap, A += g * kr and B += g * ki, with the sign applied once at
@@ -282,7 +282,7 @@ __device__ __forceinline__ bool degrid_unit(const JobDesc& jd,
 // plain_large: 2 CTAs 30.3 ms, 3: 23.2, 4: 20.8, 5: 22.1, 6: 23.3 (more
 // warps share the same L1 for their kernel rows and grid lines).
 template <typename GT, typename KT>
-__global__ void __launch_bounds__(kDegridWarps * 32, 4)
+__global__ void __launch_bounds__(kDegridWarps * 32, kDegridResident)
 degrid_kernel(const uint32_t* __restrict__ order,
               const uint32_t* __restrict__ sorted_keys,
               const uint2* __restrict__ rec, const JobDesc* __restrict__ jobs,
@@ -519,20 +519,7 @@ cudaError_t launch_degrid(const uint32_t* order, const uint32_t* sorted_keys,
                           int data_is_double, int kernel_type, int num_sms,
                           cudaStream_t st)
 {
-    // Chunks of 256 share most; fewer than the 4 resident CTAs per SM leave
-    // SMs idle, so small calls take 128, 64 or 32: 23 thousand FP64 points,
-    // supports 5 to 30, 450 -> 213 us a call.  Below 8 chunks of 256 per
-    // resident CTA, the last chunks of a wide support are waited for, so there
-    // a chunk's taps are bounded too: 531 thousand points, supports 4 to 34,
-    // 583 us with 256, 485 with 128, 448 with 32; at narrow supports (242
-    // thousand points, 4 to 16) 64 instead of 256 cost 129 -> 149 us.
-    const int w = 2 * max_support + 1;
-    const size_t resident = (size_t)num_sms * 4;
-    int chunk = kDegridChunk;
-    while (chunk > 32 &&
-           (n < resident * chunk ||
-            (n < resident * 8 * kDegridChunk && chunk * w * w > 300000)))
-        chunk /= 2;
+    const int chunk = degrid_chunk(n, max_support, data_is_double, num_sms);
     // up to 8 CTAs of 8 warps per SM, persistent over the work queue
     const size_t want = (n + chunk - 1) / chunk;
     const size_t cap = (size_t)num_sms * 8;
