@@ -280,8 +280,8 @@ __device__ __forceinline__ KT load_kernel(const KT* p)
     else return *p;
 }
 
-template <typename GT, typename KT, int CPT, bool COUNT, bool GMEM,
-          typename FL>
+template <typename GT, typename KT, int CPT, bool STRAIGHT, bool COUNT,
+          bool GMEM, typename FL>
 __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vis,
                                              int m, int w, int pitch,
                                              int row_shift,
@@ -312,21 +312,17 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
         // at plain_large without it); masked slots never flush.
         using Acc = typename FL::Acc;
         Acc acc[CPT];                       // (re, im) of each row's cell
-        // Of each slot: its footprint row, or (kStraight) its cell.
+        // Of each slot: its footprint row, or (STRAIGHT) its cell.
         unsigned at[CPT];
         constexpr bool kFused =
             std::is_same<FL, PlainFlush<float>>::value && !COUNT;
-        // Most visibilities have the cell of the one before (tasks hold all
-        // planes of a support, in cell order): their classes stay where they
-        // are, and a branch the whole warp takes skips the row wrap, the cell
-        // arithmetic and the flush.  What counts is that the loads still come
-        // before the flush.  Gridding, straight-line code (two visibilities
-        // per iteration) -> with the branch: 39.2 M points 16.38 -> 15.57 ms,
-        // 2.2 M 510 -> 481 us, 24 channels 2560 -> 2412, FP64 1.9 M 1886 ->
-        // 1692; with the flush before the loads 17.7 ms.  FP64 sums of FP32
-        // data need more registers than that leaves (5.06 -> 7.8 ms), so
-        // they keep the straight-line form.
-        constexpr bool kStraight = sizeof(Acc) != sizeof(typename Vec2<GT>::type);
+        // In dense tasks most visibilities have the cell of the one before
+        // (tasks hold all planes of a support, in cell order): their classes
+        // stay where they are, and a branch the whole warp takes skips the row
+        // wrap, the cell arithmetic and the flush.  What counts is that the
+        // loads still come before the flush (after it, 39.2 M points 15.6 ->
+        // 17.7 ms).  STRAIGHT has no such branch and takes two visibilities
+        // per iteration.
         unsigned origin = s_vis[i0].origin, ru, cell0;
         {
             const unsigned mu = s_vis[i0].mu, xb = (unsigned)(b0 + s_vis[i0].mv);
@@ -336,16 +332,16 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
             for (int q = 0; q < CPT; ++q)
             {
                 at[q] = min(xb + q, xb + q - (unsigned)w);
-                if (kStraight) at[q] = cell0 + at[q] * (unsigned)grid_size;
+                if (STRAIGHT) at[q] = cell0 + at[q] * (unsigned)grid_size;
                 acc[q].x = acc[q].y = 0;
             }
         }
-#pragma unroll (kStraight ? 2 : 1)
+#pragma unroll (STRAIGHT ? 2 : 1)
         for (int i = i0; i < i1; ++i)
         {
             const TapVis<GT> v = s_vis[i];
             // (a + mu) mod W for a + mu in [0, 2W): min over unsigned wraps
-            const bool moved = kStraight || v.origin != origin;
+            const bool moved = STRAIGHT || v.origin != origin;
             unsigned rvn[CPT];
             if (moved)
             {
@@ -384,7 +380,7 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
                 for (int q = 0; q < CPT; ++q)
                 {
                     const unsigned cur =
-                        kStraight ? at[q] : cell0 + at[q] * (unsigned)grid_size;
+                        STRAIGHT ? at[q] : cell0 + at[q] * (unsigned)grid_size;
                     const unsigned cell = cell1 + rvn[q] * (unsigned)grid_size;
                     if constexpr (kFused)
                         flush.flush_reset(q >= skip, cell, cur, acc[q].x,
@@ -397,7 +393,7 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
                         acc[q].x = change ? 0 : acc[q].x;
                         acc[q].y = change ? 0 : acc[q].y;
                     }
-                    at[q] = kStraight ? cell : rvn[q];
+                    at[q] = STRAIGHT ? cell : rvn[q];
                 }
                 cell0 = cell1;
             }
@@ -413,13 +409,14 @@ __device__ __forceinline__ void process_task(const TapVis<GT>* __restrict__ s_vi
 #pragma unroll
         for (int q = 0; q < CPT; ++q)
             flush(q >= skip,
-                  kStraight ? at[q] : cell0 + at[q] * (unsigned)grid_size,
+                  STRAIGHT ? at[q] : cell0 + at[q] * (unsigned)grid_size,
                   acc[q].x, acc[q].y);
         if (COUNT) flushes += CPT - skip;
     }
 }
 
-template <typename GT, typename KT, bool COUNT, bool GMEM, typename FL>
+template <typename GT, typename KT, bool STRAIGHT, bool COUNT, bool GMEM,
+          typename FL>
 __device__ __forceinline__ void dispatch_cpt(int cpt, const TapVis<GT>* s_vis,
                                              int m, int w, int pitch,
                                              int row_shift, const KT* slab,
@@ -427,8 +424,8 @@ __device__ __forceinline__ void dispatch_cpt(int cpt, const TapVis<GT>* s_vis,
                                              unsigned& flushes)
 {
 #define B200_CPT(C)                                                         \
-    process_task<GT, KT, C, COUNT, GMEM, FL>(s_vis, m, w, pitch, row_shift, \
-                                             slab, fl, grid_size, flushes)
+    process_task<GT, KT, C, STRAIGHT, COUNT, GMEM, FL>(                     \
+        s_vis, m, w, pitch, row_shift, slab, fl, grid_size, flushes)
     // A row group never has more rows than the footprint (W = 1, 3, 5
     // take CPT = W).
     if (cpt > w) cpt = w;
@@ -442,6 +439,38 @@ __device__ __forceinline__ void dispatch_cpt(int cpt, const TapVis<GT>* s_vis,
     default: B200_CPT(5); break;
     }
 #undef B200_CPT
+}
+
+// moving: most tap records of the task lie at another cell than the one before.
+// FP32 sums of FP32 data then take the straight-line code, else the code with
+// the branch (see process_task).  Gridding with the branch everywhere, moving
+// above a half, straight-line code everywhere:
+//   39.2 M points on 8192^2, dense core        12.2, 12.0, 12.7 ms
+//   24 channels on 2048^2                      2.27, 2.27, 2.35 ms
+//   1.2 M spread over 3682^2, FP16, S 6..34    1.71, 1.46, 1.46 ms
+//   20 x 0.42 M spread over 2048^2, S 6..34    5.63, 5.26, 5.35 ms
+// A quarter or 0.7 instead of a half: 12.1 and 12.1 ms in the first, 5.31 and
+// 5.30 in the last.  FP64 data always has the branch: it gains in dense tasks
+// (1.9 M points 1799 -> 1631 us) and loses nothing in spread ones.  FP64 sums of
+// FP32 data need more registers than it leaves (5.06 -> 7.8 ms).
+template <typename GT, typename KT, bool COUNT, bool GMEM, typename FL>
+__device__ __forceinline__ void dispatch_task(bool moving, int cpt,
+                                              const TapVis<GT>* s_vis, int m,
+                                              int w, int pitch, int row_shift,
+                                              const KT* slab, const FL& fl,
+                                              int grid_size, unsigned& flushes)
+{
+    constexpr bool kFp64Data = std::is_same<GT, double>::value;
+    constexpr bool kFp64Sums = std::is_same<typename FL::Acc, double2>::value;
+    if constexpr (!kFp64Data)
+        if (kFp64Sums || moving)
+            return dispatch_cpt<GT, KT, true, COUNT, GMEM>(
+                cpt, s_vis, m, w, pitch, row_shift, slab, fl, grid_size,
+                flushes);
+    if constexpr (kFp64Data || !kFp64Sums)
+        dispatch_cpt<GT, KT, false, COUNT, GMEM>(cpt, s_vis, m, w, pitch,
+                                                 row_shift, slab, fl,
+                                                 grid_size, flushes);
 }
 
 template <typename GT, bool COMP> struct FlushFor { using type = PlainFlush<GT>; };
@@ -488,6 +517,7 @@ romein_grid_kernel(const GridArgs a)
         int total;        // its points; -1: no task is left
         int done;         // points gathered
         int pending;      // merged points of the batch in s_raw
+        int moves;        // tap records at another cell than the one before
         uint2 point;      // record of one of its points
     } s_task;
     __shared__ uint32_t s_order[kGridThreads];
@@ -495,6 +525,7 @@ romein_grid_kernel(const GridArgs a)
     __shared__ bool s_head[kTaskMax + 1];
     __shared__ int4 s_box[kGridThreads / 32];
     __shared__ int s_warp_heads[kGridThreads / 32];
+    __shared__ int s_warp_moves[kGridThreads / 32];
 
     unsigned long long* status = &a.counters[CNT_STATUS];
     const unsigned num_tasks = tasks_listed(a.counters);
@@ -523,6 +554,7 @@ romein_grid_kernel(const GridArgs a)
         // Every thread has finished with the records, the row block and the
         // task before they are overwritten below.
         __syncthreads();
+        if (t == 0) s_task.moves = 0;
         if (t == 0 && s_task.pending == 0 && s_task.done == s_task.total)
         {
             const unsigned long long task = first + atomicAdd(queue, 1ull);
@@ -620,19 +652,25 @@ romein_grid_kernel(const GridArgs a)
                 // Points with the same record read the same kernel values
                 // into the same cells: the first of each run stands for
                 // it with the sum of their visibilities.
-                bool head = false;
+                bool head = false, move = false;
                 if (t < m)
                 {
                     const uint2 r = s_raw[key & 0xffu].rec;
                     const uint2 q =
                         s_raw[s_order[t ? t - 1 : 0] & 0xffu].rec;
-                    head = t == 0 || r.x != q.x || r.y != q.y;
+                    move = t == 0 || r.x != q.x;
+                    head = move || r.y != q.y;
                 }
                 // (the end of the batch ends its last run)
                 s_head[t] = head || t >= m;
                 if (t == 0) s_head[kTaskMax] = true;
                 const unsigned ball = __ballot_sync(0xffffffffu, head);
-                if ((t & 31) == 0) s_warp_heads[t >> 5] = __popc(ball);
+                const unsigned moved = __ballot_sync(0xffffffffu, move);
+                if ((t & 31) == 0)
+                {
+                    s_warp_heads[t >> 5] = __popc(ball);
+                    s_warp_moves[t >> 5] = __popc(moved);
+                }
                 __syncthreads();
                 for (int wi = 0; wi < kGridThreads / 32; ++wi)
                     pending += s_warp_heads[wi];
@@ -662,6 +700,9 @@ romein_grid_kernel(const GridArgs a)
                                     jd.oversample, jd.half, status);
             }
             const uint32_t key = s_order[t];
+            if (t == 0)
+                for (int wi = 0; wi < kGridThreads / 32; ++wi)
+                    s_task.moves += s_warp_moves[wi];
             __syncthreads();   // the raw batch is read
             if (head) s_vis[pos] = tv;
             if (STAGED)
@@ -713,8 +754,9 @@ romein_grid_kernel(const GridArgs a)
         const auto fl = make_flush<GT, COMP>(jd, a.comp_part, comp_here);
         if (!STAGED)
         {
-            dispatch_cpt<GT, KT, COUNT, true>(cpt, s_vis, count, w, d.pitch, 0,
-                                        slabs, fl, grid_size, flushes);
+            dispatch_task<GT, KT, COUNT, true>(2 * s_task.moves > count, cpt,
+                                               s_vis, count, w, d.pitch, 0,
+                                               slabs, fl, grid_size, flushes);
             continue;
         }
         const unsigned block_elems = (unsigned)w * (unsigned)d.pitch;
@@ -746,9 +788,9 @@ romein_grid_kernel(const GridArgs a)
                 return;
             }
             phase ^= 1u;
-            dispatch_cpt<GT, KT, COUNT, false>(cpt, s_vis + rb, re - rb, w,
-                                        d.pitch, ov * (int)block_elems,
-                                        s_block, fl, grid_size, flushes);
+            dispatch_task<GT, KT, COUNT, false>(
+                2 * s_task.moves > count, cpt, s_vis + rb, re - rb, w, d.pitch,
+                ov * (int)block_elems, s_block, fl, grid_size, flushes);
             __syncthreads();
         }
     }
