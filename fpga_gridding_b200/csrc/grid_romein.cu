@@ -638,7 +638,8 @@ romein_grid_kernel(const GridArgs a)
                     if (t == 0) s_task.point = rv.rec;
                     rec = unpack_record(rv.rec);
                 }
-                const TaskKey tk(jd.half, task_box(t < m, rec, s_box));
+                const TaskKey tk(jd.half, task_box(t < m, rec, s_box),
+                                 sizeof(GT) == 8 ? m : 0);
                 uint32_t key = 0xffffffffu;
                 if (t < m) key = tk.template make<!STAGED>(rec, t);
                 // Order the batch (see TaskKey): consecutive points are
