@@ -17,9 +17,9 @@
 //     each of them,
 //   - two different ones of the same cell and support are gathered together,
 //     sharing the grid loads.
-// 15.7 M points on 8192^2 (8.0e9 taps): 8.60 -> 7.17 ms, without pairs 8.7, with
-// pairs to a width of 32 only 7.4, chunks in Morton order instead of column by
-// column 7.4; 0.24 M points in dense cells 119 -> 48 us.
+// 15.7 M points on 8192^2 (8.0e9 taps): 8.60 -> 7.17 ms, without pairs 8.7,
+// chunks in Morton order instead of column by column 7.4; 0.24 M points in dense
+// cells 119 -> 48 us.
 // A group of 16 lanes takes one or two visibilities (two groups per warp): its
 // lanes walk the footprint's taps in row-major order, 16 at a time (busy
 // whatever the support; the per-visibility set-up and reduction serve both
@@ -47,7 +47,14 @@ constexpr int kDegridWarps = 8;     // warps per CTA
 constexpr int kGroup = 16;          // lanes per visibility
 constexpr int kGroups = 32 / kGroup;
 constexpr int kDegridMaxW = 255;   // footprint width for support <= 127
-constexpr int kPairMaxW = 48;      // widest footprint gathered in pairs
+// Widest footprint gathered in pairs: in wider ones the two walks' kernel rows
+// crowd each other out of L1 where points are spread.  Pairs to a width of 24,
+// 32, 40, 48 (no pairs), FP32: 15.7 million points on 8192^2, oversample 4, 6.84,
+// 6.65, 6.71, 6.77 ms (7.52); 3.9 million spread over 4096^2, oversample 8, 4.12,
+// 4.05, 4.24, 4.45 (4.24), FP64 8.57, 8.59, 9.01, 9.15 (8.23).  33 is as good as
+// 32 (6.66 and 4.09 ms) and the first width with three columns per lane: without
+// that walk for pairs the compiled kernel takes 7.19 and 4.31 ms.
+constexpr int kPairMaxW = 33;
 
 // Sum over taps of grid * conj(Kt), Kt = (kr, sgn * ki).  FP32: two packed
 // FMAs per tap, A += g * kr and B += g * ki, with the sign applied once at
@@ -251,6 +258,7 @@ __device__ __forceinline__ bool degrid_unit(const JobDesc& jd,
     case 1: degrid_rows<1, P, GT>(slab, grid, W, pitch, G, cm, gl, acc); break;
     case 2: degrid_rows<2, P, GT>(slab, grid, W, pitch, G, cm, gl, acc); break;
     case 3: degrid_rows<3, P, GT>(slab, grid, W, pitch, G, cm, gl, acc); break;
+    // (pairs are no wider: kPairMaxW)
     case 4:
         if constexpr (P == 1)
         {
