@@ -17,9 +17,10 @@ constexpr int kDegridResident = 4;     // CTAs per SM that run at once
 //   - while the taps of one chunk at the widest support exceed a share of the
 //     call that goes with its points: such chunks, last in the queue, are
 //     waited for.  Three quarters of a tap per point, 0.6 in FP64, on 148 SMs,
-//     and never below 250 thousand taps.
+//     and never below 300 thousand taps.
 // Chunks of 256 / 128 / 64 / 32 (the rule's in brackets):
-//   FP32, 301 thousand points, supports 4 to 36    387  293 [286] 325 us
+//   FP32, 242 thousand points, supports 4 to 16   [112] 115 us (a call)
+//   FP32, 301 thousand points, supports 4 to 36    387  293  286 [325] us
 //   FP32, 1.0 M, supports 4 to 36                  550 [518] 600  758 us
 //   FP32, 1.0 M, supports 4 to 24                 [409] 409  473  615 us
 //   FP32, 1.3 M, supports 4 to 127                6.19 5.03 4.73 [4.89] ms
@@ -30,7 +31,7 @@ constexpr int kDegridResident = 4;     // CTAs per SM that run at once
 inline int degrid_chunk(size_t n, int max_support, bool is_double, int num_sms)
 {
     const double w = 2.0 * max_support + 1.0;
-    const double most = std::max(250000.0, (is_double ? 0.6 : 0.75) * (double)n);
+    const double most = std::max(300000.0, (is_double ? 0.6 : 0.75) * (double)n);
     const size_t resident = (size_t)num_sms * kDegridResident;
     int chunk = kDegridChunk;
     while (chunk > kDegridChunkMin &&

@@ -25,7 +25,7 @@ def _points(chunk, support, single):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     taps = chunk * (2 * max(support) + 1) ** 2
     n = 4 * sms * chunk
-    if taps > 250000:
+    if taps > 300000:
         n = max(n, math.ceil(taps / (0.75 if single else 0.6)))
     return n + 13
 
