@@ -453,7 +453,10 @@ __device__ __forceinline__ void dispatch_cpt(int cpt, const TapVis<GT>* s_vis,
 // 5.30 in the last.  FP64 data always has the branch: it gains in dense tasks
 // (1.9 M points 1799 -> 1631 us) and loses nothing in spread ones.  FP64 sums of
 // FP32 data need more registers than it leaves (5.06 -> 7.8 ms).
-template <typename GT, typename KT, bool COUNT, bool GMEM, typename FL>
+// BOTH false: the branch only, in a kernel half as long, for calls of so few
+// points that its start counts (10 thousand: 17.0 us against 17.9 with both).
+template <typename GT, typename KT, bool BOTH, bool COUNT, bool GMEM,
+          typename FL>
 __device__ __forceinline__ void dispatch_task(bool moving, int cpt,
                                               const TapVis<GT>* s_vis, int m,
                                               int w, int pitch, int row_shift,
@@ -462,7 +465,7 @@ __device__ __forceinline__ void dispatch_task(bool moving, int cpt,
 {
     constexpr bool kFp64Data = std::is_same<GT, double>::value;
     constexpr bool kFp64Sums = std::is_same<typename FL::Acc, double2>::value;
-    if constexpr (!kFp64Data)
+    if constexpr (!kFp64Data && (kFp64Sums || BOTH))
         if (kFp64Sums || moving)
             return dispatch_cpt<GT, KT, true, COUNT, GMEM>(
                 cpt, s_vis, m, w, pitch, row_shift, slab, fl, grid_size,
@@ -491,7 +494,8 @@ make_flush(const JobDesc& jd, int comp_part, bool active)
 // At least grid_ctas_per_sm<GT>() CTAs per SM, with at most 6 rows per thread.
 // 39.2 M FP32 points: 4 CTAs (64 registers) 15.6 ms, 3 16.6, 5 16.2.  1.9 M
 // FP64 points: 3 CTAs (80 registers) 1692 us, 2 1860, 4 2406 (spills).
-template <typename GT, typename KT, bool STAGED, bool COMP, bool COUNT>
+template <typename GT, typename KT, bool STAGED, bool COMP, bool COUNT,
+          bool BOTH>
 __global__ void __launch_bounds__(kGridThreads, grid_ctas_per_sm<GT>())
 romein_grid_kernel(const GridArgs a)
 {
@@ -507,6 +511,8 @@ romein_grid_kernel(const GridArgs a)
                                             sizeof(TapVis<GT>) - 1) /
                                            sizeof(TapVis<GT>));
     RawVis<GT>* s_raw = reinterpret_cast<RawVis<GT>*>(s_vis + kKeep);
+    // (see dispatch_task; the others have one loop, and nothing to count for it)
+    constexpr bool kBoth = BOTH && sizeof(GT) == 4 && !COMP;
     __shared__ uint64_t s_bar;
     // The CTA's task: what is left of it when the classes run (kept here and
     // not in registers, which the tap loop needs).
@@ -554,7 +560,7 @@ romein_grid_kernel(const GridArgs a)
         // Every thread has finished with the records, the row block and the
         // task before they are overwritten below.
         __syncthreads();
-        if (t == 0) s_task.moves = 0;
+        if (kBoth && t == 0) s_task.moves = 0;
         if (t == 0 && s_task.pending == 0 && s_task.done == s_task.total)
         {
             const unsigned long long task = first + atomicAdd(queue, 1ull);
@@ -666,11 +672,11 @@ romein_grid_kernel(const GridArgs a)
                 s_head[t] = head || t >= m;
                 if (t == 0) s_head[kTaskMax] = true;
                 const unsigned ball = __ballot_sync(0xffffffffu, head);
-                const unsigned moved = __ballot_sync(0xffffffffu, move);
-                if ((t & 31) == 0)
+                if ((t & 31) == 0) s_warp_heads[t >> 5] = __popc(ball);
+                if (kBoth)
                 {
-                    s_warp_heads[t >> 5] = __popc(ball);
-                    s_warp_moves[t >> 5] = __popc(moved);
+                    const unsigned moved = __ballot_sync(0xffffffffu, move);
+                    if ((t & 31) == 0) s_warp_moves[t >> 5] = __popc(moved);
                 }
                 __syncthreads();
                 for (int wi = 0; wi < kGridThreads / 32; ++wi)
@@ -701,7 +707,7 @@ romein_grid_kernel(const GridArgs a)
                                     jd.oversample, jd.half, status);
             }
             const uint32_t key = s_order[t];
-            if (t == 0)
+            if (kBoth && t == 0)
                 for (int wi = 0; wi < kGridThreads / 32; ++wi)
                     s_task.moves += s_warp_moves[wi];
             __syncthreads();   // the raw batch is read
@@ -755,9 +761,9 @@ romein_grid_kernel(const GridArgs a)
         const auto fl = make_flush<GT, COMP>(jd, a.comp_part, comp_here);
         if (!STAGED)
         {
-            dispatch_task<GT, KT, COUNT, true>(2 * s_task.moves > count, cpt,
-                                               s_vis, count, w, d.pitch, 0,
-                                               slabs, fl, grid_size, flushes);
+            dispatch_task<GT, KT, kBoth, COUNT, true>(
+                kBoth && 2 * s_task.moves > count, cpt, s_vis, count, w, d.pitch, 0,
+                slabs, fl, grid_size, flushes);
             continue;
         }
         const unsigned block_elems = (unsigned)w * (unsigned)d.pitch;
@@ -789,8 +795,8 @@ romein_grid_kernel(const GridArgs a)
                 return;
             }
             phase ^= 1u;
-            dispatch_task<GT, KT, COUNT, false>(
-                2 * s_task.moves > count, cpt, s_vis + rb, re - rb, w, d.pitch,
+            dispatch_task<GT, KT, kBoth, COUNT, false>(
+                kBoth && 2 * s_task.moves > count, cpt, s_vis + rb, re - rb, w, d.pitch,
                 ov * (int)block_elems, s_block, fl, grid_size, flushes);
             __syncthreads();
         }
@@ -804,11 +810,11 @@ romein_grid_kernel(const GridArgs a)
 }
 
 template <typename GT, typename KT, bool STAGED, bool COMP = false,
-          bool COUNT = false>
+          bool COUNT = false, bool BOTH = true>
 cudaError_t launch_variant(const GridArgs& a, int num_sms, size_t smem,
                            cudaStream_t st, int* ctas_out)
 {
-    auto fn = romein_grid_kernel<GT, KT, STAGED, COMP, COUNT>;
+    auto fn = romein_grid_kernel<GT, KT, STAGED, COMP, COUNT, BOTH>;
     // Function attributes and occupancy are looked up once per (variant,
     // device, shared-memory size), not on every launch.
     static std::mutex mu;
@@ -978,6 +984,16 @@ cudaError_t launch_grid(const GridArgs& a, int data_is_double,
         return count ? launch_variant<double, double2, false, false, true>(args, num_sms, smem, st, ctas_out)
                      : launch_variant<double, double2, false>(args, num_sms, smem, st, ctas_out);
     }
+    if (a.few_points && !staged && !count)
+        switch (kernel_type)
+        {
+        case OSKAR_B200_KERNEL_F16:
+            return launch_variant<float, __half2, false, false, false, false>(args, num_sms, smem, st, ctas_out);
+        case OSKAR_B200_KERNEL_BF16:
+            return launch_variant<float, __nv_bfloat162, false, false, false, false>(args, num_sms, smem, st, ctas_out);
+        default:
+            return launch_variant<float, float2, false, false, false, false>(args, num_sms, smem, st, ctas_out);
+        }
     switch (kernel_type)
     {
     case OSKAR_B200_KERNEL_F16:

@@ -13,6 +13,7 @@ template <typename GT>
 constexpr int grid_ctas_per_sm() { return sizeof(GT) == 8 ? 3 : 4; }
 constexpr int kTaskMax = 256;       // tap records (merged points) at a time
 constexpr int kTaskRaw = 1024;      // points per task (staged: kTaskMax)
+constexpr size_t kFewPoints = size_t(1) << 14;   // see GridArgs::few_points
 constexpr int kTuneMax = 128;       // supports covered by the tune table
 constexpr unsigned kBulkChunk = 32768;  // bytes per cp.async.bulk
 constexpr int kMaxOffsets = 33;     // 2 * ceil(oversample / 2) + 1, oversample <= 32
@@ -22,6 +23,8 @@ struct GridArgs
     const uint32_t* order;      // sorted position -> point (global index)
     const uint2* rec;           // placement record of each point
     int apply_weight;           // visibilities x weight (see JobDesc)
+    int few_points;             // at most kFewPoints in the call: the shorter
+                                // kernel (see dispatch_task)
     const uint32_t* task_start; // [num_tasks + 1]
     const uint32_t* task_job;   // [num_tasks]: job of each task
     const JobDesc* jobs;        // cube, grid and geometry of each job

@@ -456,6 +456,7 @@ int run_batch(oskar_B200Workspace* ws, const oskar_B200Options* opt,
     ga.order = vals[which];
     ga.rec = pa.rec;
     ga.apply_weight = opt->apply_weight;
+    ga.few_points = n <= kFewPoints;
     ga.task_start = static_cast<const uint32_t*>(ws->task_start.ptr);
     ga.task_job = static_cast<const uint32_t*>(ws->task_job.ptr);
     ga.jobs = d_jobs;

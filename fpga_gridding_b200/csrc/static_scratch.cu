@@ -237,6 +237,7 @@ extern "C" int oskar_b200_grid_f_static(
     ga.order = vals[which];
     ga.rec = rec;
     ga.apply_weight = 0;
+    ga.few_points = n <= kFewPoints;
     ga.task_start = task_start;
     ga.task_job = task_job;
     ga.jobs = d_job;

@@ -2,7 +2,8 @@
 cell of the one before, or straight where most lie at another cell: one, two
 and three different placements per cell (all move, half of them, a third), a
 mixture of them in one call, narrow to wide footprints, kernel values through
-L1 and staged, against the CPU oracle (FP32: relative RMS <= 1e-5, FP64:
+L1 and staged, calls small enough for the kernel with the branch alone and larger
+ones, against the CPU oracle (FP32: relative RMS <= 1e-5, FP64:
 <= 1e-12)."""
 import numpy as np
 import pytest
@@ -16,12 +17,13 @@ pytestmark = pytest.mark.gpu
 G, OS = 700, 8
 
 
+@pytest.mark.parametrize("cells", [1500, 17000])
 @pytest.mark.parametrize("kw", [{}, dict(staging=1),
                                 dict(accum_mode=_lib.ACCUM_COMPENSATED)])
 @pytest.mark.parametrize("single", [False, True])
 @pytest.mark.parametrize("per_cell", [(1,), (2,), (3,), (1, 3), (1, 2, 3)])
 @pytest.mark.parametrize("support", [[0], [1], [2, 2], [8, 8, 3], [30, 30]])
-def test_tasks(oracle, support, per_cell, single, kw):
+def test_tasks(oracle, support, per_cell, single, kw, cells):
     if kw.get("accum_mode") and not single:
         kw = dict(classes_per_thread=4)      # (compensation is FP32 only)
     if kw.get("staging") and not single and max(support) > 20:
@@ -33,7 +35,7 @@ def test_tasks(oracle, support, per_cell, single, kw):
     real = np.float32 if single else np.float64
     # distinct cells, each with so many different offsets inside it
     side = 2 * 150
-    cells = rng.choice(side * side, 1500, replace=False)
+    cells = rng.choice(side * side, cells, replace=False)
     count = np.resize(per_cell, cells.size)
     cell = np.repeat(cells, count)
     first = np.repeat(np.cumsum(count) - count, count)
