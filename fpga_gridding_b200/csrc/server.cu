@@ -136,6 +136,23 @@ struct oskar_B200Server
         return p;
     }
 
+    // Where both planes of a compensated batch's FP64 sums would exceed the
+    // budget, its workspace gets by with one, the size an error grid had
+    // (lock held, grids taken).
+    void limit_sums(oskar_B200Workspace* ws, const std::vector<HostJob>& jobs,
+                    size_t n) const
+    {
+        size_t both = 0;
+        for (const HostJob& j : jobs)
+            both += 2 * sizeof(double) * (size_t)j.grid_size * j.grid_size;
+        const size_t held = ws->comp_grid.bytes;
+        const size_t rest = oskar_b200_workspace_bytes(ws) - held;
+        const size_t grow = std::max(workspace_need(n), rest) - rest;
+        if (both > held && in_use() + grow + both - held > budget &&
+            (!ws->comp_refused || both < ws->comp_refused))
+            ws->comp_refused = both;
+    }
+
     // Frees pooled grids until `need` more bytes fit the budget.
     void trim_pool(size_t need)
     {
@@ -287,6 +304,8 @@ struct oskar_B200Server
             if (!ok && s.jobs.empty()) break;
             jobs.resize(s.jobs.size());
             cudaMemsetAsync(s.outs.ptr, 0, 16 * jobs.size(), st);
+            if (opt.accum_mode == OSKAR_B200_ACCUM_COMPENSATED)
+                limit_sums(s.ws, jobs, n);
             int rs = run_batch(s.ws, &opt, (int)jobs.size(), jobs.data(), st,
                                false, nullptr, slices);
             if (rs == OSKAR_B200_OK)
