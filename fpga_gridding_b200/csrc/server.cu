@@ -77,9 +77,10 @@ struct Slot
 // Workspace bytes a batch of n points needs (run_batch's buffers).
 size_t workspace_need(size_t n)
 {
-    // keys and indices (twice), records, task starts and jobs, and the
-    // sort's scratch: 44 bytes per point in either precision
-    return n * 44u + (8u << 20);
+    // keys and indices (twice) 16, records 8, task starts and jobs 8, the
+    // sort's and the task list's scratch 0.5 bytes per point in either
+    // precision, and some for the rounding of each buffer to 2 MiB
+    return n * 36u + (8u << 20);
 }
 
 }  // namespace
