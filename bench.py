@@ -364,16 +364,15 @@ def run_b200(args, world, rank, local):
     achieved = alg_bytes / (kernel_ms * 1e-3) / 1e9
     peak, peak_kind = measured_peaks()
     traffic = profiled_traffic()
-    # The kernel's ceiling is not HBM: ncu shows instruction issue and the
-    # latency of its kernel-value loads limiting it with DRAM nearly idle
+    # The kernel's ceiling is not HBM: ncu shows the L1 data pipe 85 % busy
+    # and 65 % of the issue slots taken, with DRAM nearly idle
     # (profiles/romein_grid_kernel_plain_large.md).  achieved/peak/frac
     # still place its algorithmic bytes against the measured HBM copy rate;
     # the L2-atomic roofline of its grid updates is in "l2_atomic".
     roofline = {"kernel": "romein_grid_kernel<float,float2,L1>",
-                "bound": "issue",
-                "bound_evidence": "ncu small case: issue slots and "
-                                  "kernel-value load latency limit it; "
-                                  "DRAM throughput about 1 %",
+                "bound": "l1",
+                "bound_evidence": "ncu, full size: L1 data pipe 85 % busy, "
+                                  "issue slots 65 %, DRAM throughput 7 %",
                 "achieved": round(achieved, 2), "peak": peak,
                 "peak_source": peak_kind, "unit": "GB/s",
                 "frac": round(achieved / peak, 4),
@@ -1255,11 +1254,10 @@ def run_degrid(args, world, rank, local):
                         "sort": round(st.sort_ms, 3),
                         "degrid": round(st.grid_ms, 3)},
            "roofline": {"kernel": "degrid_kernel<float,float2>",
-                        "bound": "issue",
-                        "bound_evidence": "ncu: L1 loads of kernel values "
-                                          "and grid cells and instruction "
-                                          "issue limit it; DRAM throughput "
-                                          "about 5 %",
+                        "bound": "l1",
+                        "bound_evidence": "ncu, full size: L1 data pipe 85 % "
+                                          "busy with kernel values and grid "
+                                          "cells; DRAM throughput 6 %",
                         "achieved": round(achieved, 2),
                         "peak": peak, "peak_source": peak_kind,
                         "unit": "GB/s", "frac": round(achieved / peak, 4),

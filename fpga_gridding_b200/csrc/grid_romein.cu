@@ -1,12 +1,12 @@
 // Romein-style W-projection scatter kernel for sm_100a.
 //
-// Work arrives as tasks: runs of <= kTaskMax sorted visibilities that share
-// a support S (hence a footprint width W = 2S+1) and a coarse grid tile; with
-// staging on, a w-plane.  A persistent CTA pulls tasks from a device work queue.  For a
-// task it
-//   0. gathers the task's placement records and visibilities through the
+// Work arrives as tasks: runs of <= kTaskRaw sorted visibilities that share a
+// support S (hence a footprint width W = 2S+1) and a coarse grid tile; with
+// staging on, runs of <= kTaskMax that share a w-plane.  A persistent CTA pulls
+// tasks from a device work queue.  For a task, in batches of kTaskMax, it
+//   0. gathers the batch's placement records and visibilities through the
 //      sort's index array (sorted position -> point),
-//   1. orders the task's visibilities by cell (and kernel row offset) and
+//   1. orders the batch's visibilities by cell (and kernel row offset) and
 //      turns each into a small tap record in shared memory, merging records
 //      whose taps are identical,
 //   2. reads kernel values through L1 (default) or, with staging on, copies
@@ -204,8 +204,8 @@ __device__ __forceinline__ TaskLayout task_layout(int w)
 // Grid flush policies.  PlainFlush: one predicated vector reduction.
 // CompensatedFlush (FP32 grids): the running sums are FP64 and go to FP64
 // planes of sums, one of the real and one of the imaginary parts, which are
-// added to the grid at the end of the job.  Every cell is then rounded to FP32
-// once.  Two fire-and-forget reductions of consecutive lanes replace the
+// rounded to FP32 once, at the end of the job, and added to the grid's value in
+// FP32.  Two fire-and-forget reductions of consecutive lanes replace the
 // returning FP32 atomic whose rounding error (Knuth's TwoSum) was collected in
 // an error grid: 3.4 M points on 4096^2, oversample 8, gridding 10.6 ->
 // 5.1 ms, error against FP64 5.3e-8 -> 3.3e-8 (FP32 running sums with these
@@ -876,7 +876,8 @@ cudaError_t launch_variant(const GridArgs& a, int num_sms, size_t smem,
 // column work plus ~20 per class, so the cost of a tap is
 // (12 / CPT + 20) / utilisation, utilisation being the fraction of the
 // CTA's thread slots (threads x CPT x passes) holding a live class under
-// the (column, row group) layout of process_task.
+// the (column, row group) layout of process_task.  (Modelled on FP32 sums; FP64
+// data and FP64 sums, twice as wide in registers, take the same table.)
 void default_tune_table(unsigned char* cpt)
 {
     const int choices[] = {1, 2, 3, 4, 5, 6};

@@ -19,7 +19,11 @@ namespace b200 {
 // 24 / 32 bits: 10 thousand points, sort 30 / 38 / 38 us, gridding 16 us each;
 // 0.24 M, 32 / 46 / 57 and 68 / 45 / 45 us; 2.2 M, 77 / 108 / 136 and 703 /
 // 541 / 508 us, error against FP64 1.5e-6 with 24 bits, 0.65e-6 with 32;
-// 39.2 M, 0.70 / 1.04 / 1.36 and 29.4 / 18.8 / 16.2 ms.
+// 39.2 M, 0.70 / 1.04 / 1.36 and 29.4 / 18.8 / 16.2 ms.  (Single jobs.  The job
+// field of a batch comes out of the same bits: against the build before, which
+// always had 31, batches of 16 to 200 jobs of 1 to 60 thousand points take 0.74
+// to 0.92 of the time, with errors of 0.70 to 1.03; the lines were not measured
+// for batches by themselves.)
 static int key_bits(size_t num_points)
 {
     return num_points <= (size_t(1) << 14)   ? 16

@@ -170,8 +170,9 @@ struct PrepArgs
 // Blocks per job: about 8 per SM over the whole batch, at least one per job,
 // no more than the largest job needs.
 int prep_blocks_per_job(size_t max_points, int num_jobs, int num_sms);
-// The last block of each job adds the job's partials to its norm and publishes
-// its skip count and grid updates.  (Also for jobs without points.)
+// Every block adds its grid updates to the counters; the last block of each job
+// adds the job's partials to its norm and publishes its skip count.  (Also for
+// jobs without points.)
 cudaError_t launch_prep(const PrepArgs& a, int data_is_double, int coord_mode,
                         cudaStream_t st);
 // Task list: a task starts where (job, coarse tile, group) changes and every

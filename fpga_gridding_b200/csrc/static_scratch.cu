@@ -16,7 +16,7 @@
 // entry point runs on each device (with that device current) and cached.
 // That first call must therefore not happen inside a stream capture.
 // Every call uses the same array, and it keeps the previous call's
-// contents: the counters and histograms are cleared each call, and two
+// contents: the counters and the sort's scratch are cleared each call, and two
 // calls whose work overlaps on the GPU (different streams, or different
 // threads) race on the array, so callers must serialise them.
 #include <algorithm>
@@ -39,7 +39,7 @@ int static_cube_fill(const float* d_conv, int num_planes, int oversample,
 
 namespace {
 
-// 64 MiB: about 1.5 million visibilities with a small cube (~41 bytes of
+// 64 MiB: about 2 million visibilities with a small cube (~33 bytes of
 // scratch per visibility plus the re-laid cube).
 constexpr size_t kStaticScratchBytes = size_t(64) << 20;
 constexpr int kMaxDevices = 64;
@@ -228,6 +228,8 @@ extern "C" int oskar_b200_grid_f_static(
     B200_S(radix_sort_pairs(keys, vals, n, kl.total_bits + 1, sort_tmp,
                             counters + CNT_STATUS, num_sms, s, &which,
                             nullptr));
+    // One batch per task at every support: the tap limits and longer tasks of
+    // the other entry points (task_sizes) were not measured here.
     TaskSizes sizes{};
     while ((1 << sizes.log2_max[0]) < kTaskMax) ++sizes.log2_max[0];
     B200_S(launch_tasks(keys[which], n, counters, 2 * kl.fine_bits,

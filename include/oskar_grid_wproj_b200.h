@@ -214,13 +214,15 @@ enum
 };
 
 /* Grid accumulation for FP32 data.  COMPENSATED: the job's contributions are
- * summed in FP64 (two planes of grid_size^2 doubles in the workspace; one
- * plane and two runs over the points where both do not fit) and added to the
- * grid once, at the end. */
+ * summed in FP64, rounded to FP32 once per cell at the end and added to the
+ * grid.  The sums take 16 bytes per cell of workspace (two planes of
+ * grid_size^2 doubles), cleared and read by every call; 8 bytes and two runs
+ * over the points where both planes do not fit.  A size that did not fit is
+ * remembered by the workspace, so later calls allocate nothing for it. */
 enum
 {
     OSKAR_B200_ACCUM_PLAIN = 0,        /* FP32 register sums, FP32 atomics */
-    OSKAR_B200_ACCUM_COMPENSATED = 1   /* FP64 sums, one rounding per cell */
+    OSKAR_B200_ACCUM_COMPENSATED = 1   /* FP64 sums, rounded once */
 };
 
 typedef struct oskar_B200Options
@@ -260,7 +262,9 @@ typedef struct oskar_B200Workspace oskar_B200Workspace;
 OSKAR_B200_EXPORT int oskar_b200_workspace_create(int device,
         oskar_B200Workspace** ws);
 OSKAR_B200_EXPORT int oskar_b200_workspace_free(oskar_B200Workspace* ws);
-/* Bytes of device memory currently held by the workspace. */
+/* Bytes of device memory currently held by the workspace: about 33 per point
+ * of the largest call, and with OSKAR_B200_ACCUM_COMPENSATED 16 (or 8) per
+ * grid cell. */
 OSKAR_B200_EXPORT size_t oskar_b200_workspace_bytes(
         const oskar_B200Workspace* ws);
 
@@ -522,7 +526,7 @@ OSKAR_B200_EXPORT int oskar_b200_measure_atomic_rate(oskar_B200Workspace* ws,
  * are device pointers; support is host memory; weight is ignored as in the
  * reference.  All scratch (the re-laid cube, sort keys, records, task list)
  * comes from one static device array of 64 MiB that every GPU loading this
- * library holds until the process exits: enough for about 1.5 million
+ * library holds until the process exits: enough for about 2 million
  * visibilities with a small cube.  A job that does not fit returns
  * OSKAR_B200_ERR_OVER_BUDGET and touches nothing.  The array's device
  * address is looked up on the first call on each device (with that device
